@@ -53,9 +53,9 @@ unsigned long long msaq_launch_count(void);
  *   launched with programmatic stream serialisation, so the launch and prologue of one kernel overlap the
  *   tail of the kernel before it.  Results do not change: every kernel waits for its predecessor before it
  *   reads or writes anything another kernel produces or consumes.
- * MSAQ_OPT_TENSOR_MEMORY (default 1): batched GEMVs (u=4, gs=2, 9 rows and more) run on the tcgen05 tensor
- *   cores with accumulators in tensor memory; 0 keeps them on the warp-level integer MMA path (the two paths
- *   agree to the output tolerance, not bit for bit).
+ * MSAQ_OPT_TENSOR_MEMORY (default 1): batched GEMVs (u=4, gs=2, 9 rows and more) run on exact bf16 operands -- up to
+ *   32 rows with warp-level MMAs on register operands, above on the tcgen05 tensor cores with accumulators in tensor
+ *   memory; 0 keeps them on the warp-level integer MMA path (the paths agree to the output tolerance, not bit for bit).
  * MSAQ_OPT_INKERNEL_STAGING (default 1): small integer-MMA GEMVs (up to four rows, no fused prologue, at most
  *   eighteen K blocks per thread block) convert their activations inside the main kernel, one launch per GEMV; 0
  *   runs the separate staging kernel in front, as all other launches do.  Same staged values either way.
@@ -85,7 +85,7 @@ int msaq_set_option(int option, int value);
 int msaq_get_option(int option);
 
 /* Status word of the current device (no reference counterpart; the reference's kernels have no waits that can
- * give up).  Bits: 1 = a wait gave up in the integer-MMA GEMV, 2 = in the tensor-memory GEMV, 4 = in the
+ * give up).  Bits: 1 = a wait gave up in a warp-level GEMV (integer or register operands), 2 = in the tensor-memory GEMV, 4 = in the
  * flash-decode kernel, 8 = an append position read from device memory was outside [0, Lcap) and the row was
  * skipped.  The call synchronises `stream`, stores the word in *status_out and, when clear != 0, resets it.
  * Do not call it while `stream` is being captured. */
@@ -98,7 +98,8 @@ int msaq_wait_status(int clear, void* stream, int* status_out);
 
 /* ------------------------------------------------------------------ GEMV -- */
 
-/* Bytes of workspace the three GEMV entry points need for these sizes. */
+/* Bytes of workspace the three GEMV entry points make use of for these sizes (some sizes also run, on a slower kernel,
+ * with less: the kernels that need the most are left out where the workspace does not hold their partial sums). */
 size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs);
 
 /*
@@ -124,7 +125,7 @@ int msaq_wonly_gemv_wide(const void* x, const int8_t* scale_exp, const uint8_t* 
 
 /*
  * Y[M,OUT] = X[M,K] . dequant(W)^T on column-major planes, any M >= 1.
- * (The tensor-memory kernel -- 9 rows and more, and the u = 2, 3 formats at gs = 2 -- widens q * 2^e through an
+ * (The tensor-memory kernel -- gs = 2, more than 32 rows -- widens q * 2^e through an
  * fp32 constant of about 2^23 * 2^e: block exponents above 104 overflow there.  bf16 weights of magnitude below
  * 2^110 never produce them.)
  * Replaces op `msaq::wonly_gemv_batched` (csrc/pybind.cpp:205-206, host

@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "gemv_mma.cuh"
+#include "gemv_reg.cuh"
 #include "gemv_umma.cuh"
 
 namespace msaq {
@@ -205,12 +206,68 @@ int run_umma(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const 
             const int64_t quads = (int64_t)rows * (OUT / 4);
             launch_chained(gemv_umma_combine_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st,
                            static_cast<const float*>(partial), static_cast<const int*>(status),
-                           static_cast<__nv_bfloat16*>(Y), Yf, sch, (int)m0, rows, (int)OUT);
+                           static_cast<__nv_bfloat16*>(Y), Yf, sch, (int)m0, rows, (int)OUT, 0);
             count_launch();
             if (int rc = check_launch("gemv_umma_combine")) return rc;
         }
     }
     return MSAQ_OK;
+}
+
+// ---- register-operand path (gs = 2, column-major planes, OUT % 16 == 0, up to 32 rows) --------------
+// Against the tensor-memory kernel, which serves what is left, us per call (rows: 1 | 16 | 32):
+//   28672x4096 u3  53.9 | 57.3 | 61.7 -> 39.5 | 44.1 | 58.8     u4, 16 | 32 rows  52.2 | 56.9 -> 38.5 | 51.3
+//   4096x4096  u3  23.3 | 26.1 | 28.5 -> 13.9 | 15.5 | 19.8     u4                25.3 | 27.5 -> 14.4 | 18.5
+//   1024x8192  u3  36.4 | 38.9        -> 10.0 | 18.0            u4                37.6        -> 17.4
+// One thread block per SM: fewer partial sums per tile than with two or three (4096x4096 u4, 16 rows: three 21.4 us, two
+// 16.7 us, one 14.4 us).
+struct RegPlan {
+    GemvSchedule sch;        // sch.nb counts units of GR_KB K blocks
+    int mt;                  // n-tiles of eight activation rows
+    size_t partial_off, total;
+};
+
+RegPlan plan_reg(int64_t M, int64_t OUT, int64_t NB, int u) {
+    RegPlan p;
+    GemvSchedule& s = p.sch;
+    const int64_t rows = M < GR_MAX_M ? M : GR_MAX_M;
+    p.mt = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
+    s.tc = GR_TC;
+    s.nb = (int)((NB + GR_KB - 1) / GR_KB);
+    s.col_tiles = (int)((OUT + GR_TC - 1) / GR_TC);
+    const long long units = s.units(), slots = sm_count();
+    s.grid = (int)(units < slots ? units : slots);
+    s.max_slots = (int)(((long long)s.nb * s.grid + units - 1) / units) + 1;
+    const int stages = (225 * 1024 - gr_merge_bytes(p.mt)) / (GR_TEAMS * gr_stage_bytes(u, p.mt));
+    s.stages = stages > GM_MAX_STAGES ? GM_MAX_STAGES : stages;
+    const size_t ctl = (256 + (size_t)s.col_tiles * GM_WARPS * sizeof(unsigned long long) + 255) & ~(size_t)255;
+    p.partial_off = ctl > WS_CTL_BYTES ? ctl : WS_CTL_BYTES;
+    p.total = p.partial_off + (((size_t)s.max_slots * rows * OUT * sizeof(float) + 255) & ~(size_t)255);
+    return p;
+}
+
+int run_reg(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y, float* Yf,
+            int64_t M, int64_t OUT, int64_t NB, int u, const RegPlan& p, void* ws, cudaStream_t st) {
+    uint8_t* base = static_cast<uint8_t*>(ws);
+    int* status = reinterpret_cast<int*>(base);
+    unsigned long long* counters = reinterpret_cast<unsigned long long*>(base + 256);
+    float* partial = reinterpret_cast<float*>(base + p.partial_off);
+    const GemvSchedule& sch = p.sch;
+    const uint32_t tag = next_call_tag();
+    // Split tiles: up to eight rows the warp that arrives last at a tile adds the partial sums up; above, it would have too
+    // many of them in hand one after another, and a second, fully parallel launch is faster (4096x4096, 16 rows: 18.2 us
+    // inside, 14.4 us with the launch; 1024x8192, eight rows: 14.0 us inside, 17.2 us with it).
+    const int combine = M > 8;
+    GemvRegArgs a{se, up, sh, X, partial, counters, status, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf, 0, (int)M,
+                  (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(), tag, combine};
+    const int rc = gemv_reg_launch(a, u, p.mt, st);
+    if (rc || !combine || (sch.units() % sch.grid == 0 && (sch.units() / sch.grid) % sch.nb == 0)) return rc;
+    const int64_t quads = M * (OUT / 4);
+    launch_chained(gemv_umma_combine_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st,
+                   static_cast<const float*>(partial), static_cast<const int*>(status), static_cast<__nv_bfloat16*>(Y), Yf,
+                   sch, 0, (int)M, (int)OUT, (int)tag);
+    count_launch();
+    return check_launch("gemv_umma_combine");
 }
 
 // Glue fused in front of the GEMV (see XprepMode); mode XP_PLAIN when absent.
@@ -324,7 +381,7 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     if (M > INT32_MAX || OUT > INT32_MAX || NB * BLOCK > INT32_MAX) return fail(MSAQ_ERR_ARG, "size exceeds 2^31");
     if (cm && (reinterpret_cast<uintptr_t>(up) & 3)) return fail(MSAQ_ERR_ARG, "upper_cm must be 4-byte aligned");
     if (int rc = require_sm100()) return rc;
-    const size_t need = msaq_wonly_gemv_workspace(M, OUT, NB, u, gs);
+    const size_t need = gemv_workspace_min(M, OUT, NB, u, gs);
     if (!ws || ws_bytes < need)
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, ws ? ws_bytes : (size_t)0);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -335,7 +392,12 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     // the tensor-memory epilogue stores 16 outputs at a time: Y (and Y_f32) must be 16-byte aligned for it
     const bool tm_ok = aligned && umma_eligible(OUT, u, gs, cm) && option_tensor_memory() &&
                        !((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15);
-    // u = 4 keeps up to eight rows on the integer-MMA kernel; the 5+3 and 6+2 bit formats have no such kernel
+    // up to 32 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
+    if (tm_ok && M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
+        const RegPlan p = plan_reg(M, OUT, NB, u);
+        if (ws_bytes >= p.total) return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, p, ws, st);
+    }
+    // u = 4 keeps up to eight rows on the integer-MMA kernel
     if (tm_ok && (u != 4 || M >= GU_MIN_M)) return run_umma(x, se, up, sh, Y, Yf, M, OUT, NB, u, ws, st);
     // the integer-MMA kernel's finishing warps store four outputs at a time: 8-byte aligned bf16, 16-byte aligned fp32
     const bool out_ok = !((reinterpret_cast<uintptr_t>(Y) & 7) | (reinterpret_cast<uintptr_t>(Yf) & 15));
@@ -350,7 +412,7 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
 
 using namespace msaq;
 
-extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
+size_t msaq::gemv_workspace_min(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
     if (M <= 0 || OUT <= 0 || NB <= 0) return 0;
     size_t bytes = gemv_generic_workspace(M, OUT, NB) + WS_CTL_BYTES;
     if (mma_eligible(OUT, u, gs, true)) {
@@ -360,6 +422,20 @@ extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, 
     if (umma_eligible(OUT, u, gs, true) && (u != 4 || M >= GU_MIN_M)) {
         const size_t tm = plan_umma(M, OUT, NB, u).total + WS_CTL_BYTES;
         if (tm > bytes) bytes = tm;
+    }
+    return bytes;
+}
+
+size_t msaq::gemv_workspace_front(int64_t M, int64_t OUT, int64_t NB, int u, int gs, size_t tail, size_t given) {
+    const size_t full = (msaq_wonly_gemv_workspace(M, OUT, NB, u, gs) + 255) & ~(size_t)255;
+    return given >= full + tail ? full : (gemv_workspace_min(M, OUT, NB, u, gs) + 255) & ~(size_t)255;
+}
+
+extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
+    size_t bytes = gemv_workspace_min(M, OUT, NB, u, gs);
+    if (bytes && umma_eligible(OUT, u, gs, true) && M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M)) {
+        const size_t reg = plan_reg(M, OUT, NB, u).total;
+        if (reg > bytes) bytes = reg;
     }
     return bytes;
 }
@@ -387,10 +463,12 @@ extern "C" int msaq_wonly_gemv_batched(const void* X, const int8_t* scale_exp, c
 }
 
 // ---- GEMV with the layer glue in front of it fused into the activation staging ---------------
+static size_t fused_tail(int64_t M, int64_t NB) { return ((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255; }
+
 extern "C" size_t msaq_wonly_gemv_fused_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
     const size_t g = msaq_wonly_gemv_workspace(M, OUT, NB, u, gs);
     if (g == 0) return 0;
-    return ((g + 255) & ~(size_t)255) + (((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255);
+    return ((g + 255) & ~(size_t)255) + fused_tail(M, NB);
 }
 
 extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* addend, int addend_is_f32, float eps,
@@ -420,7 +498,7 @@ extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* ad
     }
     if (M > INT32_MAX || OUT > INT32_MAX || NB * BLOCK > INT32_MAX / 2) return fail(MSAQ_ERR_ARG, "size exceeds 2^31");
     if (int rc = require_sm100()) return rc;
-    const size_t need = msaq_wonly_gemv_fused_workspace(M, OUT, NB, u, gs);
+    const size_t g = gemv_workspace_front(M, OUT, NB, u, gs, fused_tail(M, NB), workspace_bytes), need = g + fused_tail(M, NB);
     if (!workspace || workspace_bytes < need)
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need,
                     workspace ? workspace_bytes : (size_t)0);
@@ -436,7 +514,6 @@ extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* ad
                        workspace, st);
     }
     // Other formats: the glue runs as kernels of its own into the tail of the workspace.
-    const size_t g = (msaq_wonly_gemv_workspace(M, OUT, NB, u, gs) + 255) & ~(size_t)255;
     void* tmp = static_cast<uint8_t*>(workspace) + g;
     int rc = MSAQ_OK;
     if (prologue == MSAQ_PRO_RMSNORM) rc = msaq_rmsnorm(x, tmp, M, K, eps, stream);
@@ -460,7 +537,7 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
     if (M <= 0 || OUT <= 0 || NB <= 0) return fail(MSAQ_ERR_ARG, "M, OUT and NB must be positive");
     if (M > INT32_MAX || OUT > INT32_MAX || NB * BLOCK > INT32_MAX / 2) return fail(MSAQ_ERR_ARG, "size exceeds 2^31");
     if (int rc = require_sm100()) return rc;
-    const size_t need = msaq_wonly_gemv_fused_workspace(M, OUT, NB, u, gs);
+    const size_t need = gemv_workspace_front(M, OUT, NB, u, gs, fused_tail(M, NB), workspace_bytes) + fused_tail(M, NB);
     if (!workspace || workspace_bytes < need)
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
     const bool ok = !((reinterpret_cast<uintptr_t>(x) & 15) | (reinterpret_cast<uintptr_t>(y) & 7) |
@@ -547,7 +624,7 @@ extern "C" size_t msaq_static_scratch_bytes(void) { return MSAQ_STATIC_SCRATCH_B
 extern "C" int msaq_wonly_gemv_wide_static(const void* x, const int8_t* scale_exp, const uint8_t* upper_cm,
                                            const uint8_t* shared_cm, void* y, float* y_f32, int64_t OUT, int64_t NB,
                                            int u, int gs, void* stream) {
-    const size_t need = msaq_wonly_gemv_workspace(1, OUT, NB, u, gs);
+    const size_t need = gemv_workspace_min(1, OUT, NB, u, gs);
     if (need == 0) return msaq::fail(MSAQ_ERR_ARG, "OUT and NB must be positive");
     if (need > MSAQ_STATIC_SCRATCH_BYTES)
         return msaq::fail(MSAQ_ERR_WORKSPACE,

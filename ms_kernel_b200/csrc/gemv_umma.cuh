@@ -115,11 +115,6 @@ __host__ __device__ inline uint32_t umma_idesc_bf16(int n) {
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
 
 // ---- activation staging ----------------------------------------------------------
 // X [M][K] bf16 row-major -> per K block the first ceil(M/8) row groups of an A-operand tile in the
@@ -540,18 +535,19 @@ gemv_umma_kernel(const GemvUmmaArgs a) {
 
 // Sum of the split-K partials of the tensor-memory kernel, in slot order: one thread per four
 // consecutive outputs of one activation row.  Tiles that one CTA covered alone were written by
-// that CTA and are skipped.  A set status word (a wait gave up) marks the whole launch NaN.
+// that CTA and are skipped.  A status word that says that a wait gave up marks the whole launch NaN: the tensor-memory
+// kernel clears the word in front (tag == 0: any value counts), the register kernel leaves its call's tag there.
 __global__ void __launch_bounds__(256)
 gemv_umma_combine_kernel(const float* __restrict__ partial, const int* __restrict__ status, __nv_bfloat16* __restrict__ y,
-                         float* __restrict__ y_f32, GemvSchedule sch, int m0, int rows, int OUT) {
+                         float* __restrict__ y_f32, GemvSchedule sch, int m0, int rows, int OUT, int tag) {
     chain_release();
     chain_wait();
     const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int quads = OUT / 4;
     if (idx >= (int64_t)rows * quads) return;
-    const int m = (int)(idx / quads), col = (int)(idx % quads) * 4, c = col / GU_TR;
+    const int m = (int)(idx / quads), col = (int)(idx % quads) * 4, c = col / sch.tc;
     const int first = sch.first_cta(c), nslots = sch.last_cta(c) - first + 1;
-    const bool poison = *status != 0;
+    const bool poison = tag ? *status == tag : *status != 0;
     if (nslots == 1 && !poison) return;
     const int64_t sstride = (int64_t)rows * OUT;
     const float* src = partial + (int64_t)m * OUT + col;

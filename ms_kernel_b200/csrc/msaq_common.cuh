@@ -40,6 +40,11 @@ inline bool make_fmt(int u, int gs, Fmt* f) {
 // another never puts the counters under another kernel's partial sums.
 constexpr size_t WS_CTL_BYTES = 64 * 1024;
 
+// GEMV scratch: what a call cannot do without (with msaq_wonly_gemv_workspace bytes it may take a faster kernel), and the
+// bytes in front of a tail of `tail` bytes that leave the GEMV as much as `given` allows.
+size_t gemv_workspace_min(int64_t M, int64_t OUT, int64_t NB, int u, int gs);
+size_t gemv_workspace_front(int64_t M, int64_t OUT, int64_t NB, int u, int gs, size_t tail, size_t given);
+
 // ---- host-side error plumbing (defined in capi.cu) -------------------------
 int fail(int code, const char* fmt, ...);
 int check_launch(const char* what);

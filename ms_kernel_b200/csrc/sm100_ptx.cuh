@@ -82,6 +82,15 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
+// 16 bytes global -> shared by the calling thread, asynchronously; cp_async_arrive counts the thread's arrival on `bar` once
+// all of its copies so far have landed (the barrier's count includes it).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // D(16x8,s32) = A(16x32,s8,row) * B(32x8,s8,col) + C.
 __device__ __forceinline__ void mma_s8_16832(int (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
                                              const int (&c)[4]) {
@@ -120,6 +129,12 @@ template <int OFF>
 __device__ __forceinline__ uint32_t lds32(uint32_t base) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(base), "n"(OFF));
+    return v;
+}
+template <int OFF = 0>
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr), "n"(OFF));
     return v;
 }
 template <int OFF>

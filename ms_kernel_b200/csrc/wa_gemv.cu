@@ -93,10 +93,10 @@ extern "C" int msaq_wa_gemv_batched(const void* X, const int8_t* scale_exp, cons
                                     const uint8_t* shared_cm, void* Y, float* Y_f32, int64_t M, int64_t OUT, int64_t NB,
                                     int u, int gs, void* workspace, size_t workspace_bytes, void* stream) {
     if (M <= 0 || OUT <= 0 || NB <= 0) return fail(MSAQ_ERR_ARG, "M, OUT and NB must be positive");
-    const size_t need = msaq_wa_gemv_workspace(M, OUT, NB, u, gs);
+    const size_t tail = ((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255;
+    const size_t g = gemv_workspace_front(M, OUT, NB, u, gs, tail, workspace_bytes), need = g + tail;
     if (!workspace || workspace_bytes < need)
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
-    const size_t g = (msaq_wonly_gemv_workspace(M, OUT, NB, u, gs) + 255) & ~(size_t)255;
     void* xdq = static_cast<uint8_t*>(workspace) + g;
     if (int rc = launch_quant(X, nullptr, nullptr, xdq, M, NB * BLOCK, u, gs, stream)) return rc;
     return msaq_wonly_gemv_batched(xdq, scale_exp, upper_cm, shared_cm, Y, Y_f32, M, OUT, NB, u, gs, workspace, g, stream);

@@ -1,0 +1,91 @@
+"""GPU parity of the register-operand GEMV (csrc/gemv_reg.cuh: gs = 2, up to 32 rows) at the sizes where it can go wrong:
+one and a few K blocks (four to a ring stage, two teams), ragged tiles of 256 columns, the edges of the eight-row
+n-tiles, matrices that one thread block covers and matrices that many share -- against the float64 oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import F32_REL_FRO_TOL, MAX_ABS_REL_TOL, REL_FRO_TOL
+from oracle import msaq_oracle as orc
+from test_gpu_give_up import _short_waits, _status
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(rng, OUT, K, u, M):
+    W = orc.to_bf16((rng.standard_normal((OUT, K)) * rng.uniform(0.005, 0.08, (OUT, 1))).astype(np.float32))
+    X = orc.to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    return X, orc.pack_weight(W, u, 2)
+
+
+@pytest.mark.parametrize("u", (2, 3, 4))
+@pytest.mark.parametrize("M,OUT,K", [(1, 16, 32), (8, 240, 96), (9, 256, 160), (16, 272, 4096), (17, 528, 288), (31, 16, 8224),
+                                     (32, 1040, 1312), (33, 256, 128)])
+def test_edges(rng, u, M, OUT, K):
+    import cabi
+    X, p = _case(rng, OUT, K, u, M)
+    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    cabi.check_output(got, gotf, orc.wonly_matmul(p, X), MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+
+
+@pytest.mark.parametrize("u,M", [(2, 3), (3, 8), (4, 9), (4, 32)])
+def test_misaligned_activations_and_smallest_workspace(rng, u, M):
+    """X off a 16-byte boundary, and a workspace of the size the tensor-memory kernel needs, take that kernel: the same
+    result to fp32 rounding of the sums."""
+    import cabi
+    from ms_kernel_b200 import _lib
+    L = _lib.lib()
+    OUT, K = 4096, 512
+    X, p = _case(rng, OUT, K, u, M)
+    pd = cabi.planes_to_dev(p)
+    ref = orc.wonly_matmul(p, X)
+    buf = torch.empty(M * K + 1, dtype=torch.bfloat16, device="cuda")
+    buf[1:] = cabi.bf16_dev(X).reshape(-1)
+    got, gotf = cabi.gemv("batched", buf[1:], pd, M=M)
+    cabi.check_output(got, gotf, ref, MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+
+    full = L.msaq_wonly_gemv_workspace(M, OUT, K // 32, u, 2)
+    y = torch.empty((M, OUT), dtype=torch.bfloat16, device="cuda")
+    x = cabi.bf16_dev(X)
+    ws = torch.empty(full, dtype=torch.uint8, device="cuda")
+    served = []
+    for size in range(full, 0, -max(256, full // 64)):
+        rc = L.msaq_wonly_gemv_batched(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
+                                       pd["shared_cm"].data_ptr(), y.data_ptr(), None, M, OUT, K // 32, u, 2, ws.data_ptr(),
+                                       size, torch.cuda.current_stream().cuda_stream)
+        if rc:
+            assert rc == -3
+            break
+        served.append(y.float().cpu().numpy())
+    for s in served:
+        assert orc.rel_fro(s, got) < 1e-3           # a few roundings to bf16 at most
+
+
+def test_bits_do_not_depend_on_the_workspace_contents(rng):
+    import cabi
+    X, p = _case(rng, 1024, 2048, 3, 5)
+    pd = cabi.planes_to_dev(p)
+    x = cabi.bf16_dev(X)
+    first = cabi.gemv("batched", x, pd, M=5)[1]
+    junk = torch.randint(0, 255, (64 << 20,), dtype=torch.uint8, device="cuda")
+    del junk                                        # the next workspace comes out of these bytes
+    assert np.array_equal(cabi.gemv("batched", x, pd, M=5)[1], first)
+
+
+@pytest.mark.parametrize("u,M", [(3, 2), (4, 12)])
+def test_wait_gives_up_and_next_call_is_correct(rng, u, M):
+    import cabi
+    OUT, K = 2048, 2048
+    X, p = _case(rng, OUT, K, u, M)
+    pd = cabi.planes_to_dev(p)
+    x = cabi.bf16_dev(X)
+    ref = orc.wonly_matmul(p, X)
+    _status()
+    with _short_waits(0):
+        _, gotf = cabi.gemv("batched", x, pd, M=M)
+    assert _status() & 1
+    assert np.isnan(gotf).any()
+    got2, gotf2 = cabi.gemv("batched", x, pd, M=M)
+    cabi.check_output(got2, gotf2, ref, MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+    assert _status() == 0
