@@ -36,28 +36,97 @@ quant_act_kernel(const __nv_bfloat16* __restrict__ X, int8_t* __restrict__ qX, i
     if (Xdq) Xdq[i] = __float2bfloat16_rn((float)word * exp2_int(e));     // exact: at most 8 significant bits
 }
 
-// One thread per (output row o, block): the 32 dequantised weights as bf16 into Wbf[K][OUT] (consecutive
-// threads write consecutive o).
-__global__ void __launch_bounds__(256)
+// The 32 dequantised weights of COLS adjacent columns and one K block as bf16 into Wbf[K][OUT], consecutive threads on
+// consecutive columns.  Bound by HBM (25 to 29 bytes in, 64 out).  With the format known at compile time every field is
+// cut out with constant shifts, and a code becomes a float through the mantissa: q + 128 + 2^(u-1), which is not negative,
+// added to the bits of 2^23 reads as 2^23 plus that, and one fused multiply-add removes the offset and applies the scale
+// exactly (at most eight significant bits, so the upper half of the word is the bf16 value).  4096 x 14336 u4, us:
+// run-time shifts and an int-to-float conversion per code 160, this one (four columns, 8-byte stores) 36.
+template <int U, int LG_GS, int COLS>
+__global__ void __launch_bounds__(128)
 dequant_bf16_kernel(const int8_t* __restrict__ scale_exp, const uint8_t* __restrict__ upper_cm,
-                    const uint8_t* __restrict__ shared_cm, __nv_bfloat16* __restrict__ Wbf, int64_t OUT, Fmt f) {
+                    const uint8_t* __restrict__ shared_cm, __nv_bfloat16* __restrict__ Wbf, int64_t OUT) {
     chain_release();
     chain_wait();
-    const int64_t o = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    constexpr int WB = 8 - U, UW = WB, NG = 32 >> LG_GS, SB = (NG * U + 7) / 8;      // words of upper, bytes of shared codes
+    const int64_t o = ((int64_t)blockIdx.x * 128 + threadIdx.x) * COLS;
     const int64_t blk = blockIdx.y;
     if (o >= OUT) return;
-    const int64_t base = blk * OUT + o;
-    uint32_t uw[7], sw[3] = {0u, 0u, 0u};
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(upper_cm + base * f.UB);     // UB is a multiple of 4
+    uint32_t uw[COLS][UW + 1], sw[COLS][3];
+    float sc[COLS], off[COLS], post[COLS];
+    bool huge = false;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) uw[i] = (i * 4 < f.UB) ? src[i] : 0u;
-    uw[6] = 0u;
-    for (int i = 0; i < f.SB; ++i) sw[i >> 2] |= (uint32_t)shared_cm[base * f.SB + i] << ((i & 3) * 8);
-    const float scale = exp2_int((int)scale_exp[base]);
-#pragma unroll 4
+    for (int c = 0; c < COLS; ++c) {
+        const int64_t base = blk * OUT + o + c;
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(upper_cm + base * (4 * UW));
+#pragma unroll
+        for (int i = 0; i < UW; ++i) {
+            uint32_t flip_u = 0u;
+#pragma unroll
+            for (int b = WB - 1; b < 32 * (UW); b += WB)
+                if (b >= 32 * i && b < 32 * i + 32) flip_u |= 1u << (b - 32 * i);
+            uw[c][i] = src[i] ^ flip_u;                                              // every code offset binary
+        }
+        uw[c][UW] = 0u;
+        sw[c][0] = sw[c][1] = sw[c][2] = 0u;
+#pragma unroll
+        for (int i = 0; i < SB; ++i) sw[c][i >> 2] |= (uint32_t)shared_cm[base * SB + i] << ((i & 3) * 8);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint32_t flip_s = 0u;
+#pragma unroll
+            for (int b = U - 1; b < NG * U; b += U)
+                if (b >= 32 * i && b < 32 * i + 32) flip_s |= 1u << (b - 32 * i);
+            sw[c][i] ^= flip_s;
+        }
+        // 2^23 * 2^e overflows above e = 104: such a block is scaled in two steps
+        const int e = (int)scale_exp[base];
+        huge = huge || e > 100;
+        sc[c] = exp2_int(e > 100 ? e - 64 : e);
+        off[c] = -(8388608.0f + 128.0f + (float)(1 << (U - 1))) * sc[c];
+        post[c] = e > 100 ? 18446744073709551616.0f : 1.0f;
+    }
+    uint16_t* dst = reinterpret_cast<uint16_t*>(Wbf) + blk * BLOCK * OUT + o;
+#pragma unroll
     for (int k = 0; k < BLOCK; ++k) {
-        const int q = code_from_words(uw, k, f.wbits) * (1 << f.u) + code_from_words(sw, k >> f.lg_gs, f.u);
-        Wbf[(blk * BLOCK + k) * OUT + o] = __float2bfloat16_rn((float)q * scale);
+        uint32_t v[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            const int pu = k * WB, ps = (k >> LG_GS) * U;
+            const uint32_t fu = (pu & 31) + WB <= 32 ? uw[c][pu >> 5] >> (pu & 31)
+                                                     : __funnelshift_r(uw[c][pu >> 5], uw[c][(pu >> 5) + 1], pu & 31);
+            const uint32_t fs = (ps & 31) + U <= 32 ? sw[c][ps >> 5] >> (ps & 31)
+                                                    : __funnelshift_r(sw[c][ps >> 5], sw[c][(ps >> 5) + 1], ps & 31);
+            const uint32_t bits = ((fu & ((1u << WB) - 1u)) << U) + ((fs & ((1u << U) - 1u)) | 0x4B000000u);
+            float f = fmaf(__uint_as_float(bits), sc[c], off[c]);
+            if (huge) f *= post[c];
+            v[c] = __float_as_uint(f);
+        }
+        if constexpr (COLS == 4)
+            *reinterpret_cast<uint2*>(dst + (int64_t)k * OUT) =
+                make_uint2(__byte_perm(v[0], v[1], 0x7632), __byte_perm(v[2], v[3], 0x7632));
+        else
+            dst[(int64_t)k * OUT] = (uint16_t)(v[0] >> 16);
+    }
+}
+
+template <int U, int LG_GS>
+void launch_dequant(const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Wbf, int64_t OUT, int64_t nb, cudaStream_t st) {
+    __nv_bfloat16* w = static_cast<__nv_bfloat16*>(Wbf);
+    if (OUT % 4 == 0 && !(reinterpret_cast<uintptr_t>(Wbf) & 7))
+        launch_chained(dequant_bf16_kernel<U, LG_GS, 4>, dim3((unsigned)((OUT + 511) / 512), (unsigned)nb), dim3(128), 0, st, se, up, sh, w, OUT);
+    else
+        launch_chained(dequant_bf16_kernel<U, LG_GS, 1>, dim3((unsigned)((OUT + 127) / 128), (unsigned)nb), dim3(128), 0, st, se, up, sh, w, OUT);
+}
+
+template <int U>
+void launch_dequant_gs(const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Wbf, int64_t OUT, int64_t nb, int lg, cudaStream_t st) {
+    switch (lg) {
+        case 1: launch_dequant<U, 1>(se, up, sh, Wbf, OUT, nb, st); break;
+        case 2: launch_dequant<U, 2>(se, up, sh, Wbf, OUT, nb, st); break;
+        case 3: launch_dequant<U, 3>(se, up, sh, Wbf, OUT, nb, st); break;
+        case 4: launch_dequant<U, 4>(se, up, sh, Wbf, OUT, nb, st); break;
+        default: launch_dequant<U, 5>(se, up, sh, Wbf, OUT, nb, st); break;
     }
 }
 
@@ -117,8 +186,10 @@ extern "C" int msaq_dequant_bf16(const int8_t* scale_exp, const uint8_t* upper_c
     if (OUT <= 0 || K <= 0 || K % BLOCK) return fail(MSAQ_ERR_ARG, "K must be a positive multiple of 32");
     if (K / BLOCK > 65535) return fail(MSAQ_ERR_ARG, "K exceeds the supported range");
     if (reinterpret_cast<uintptr_t>(upper_cm) & 3) return fail(MSAQ_ERR_ARG, "upper_cm must be 4-byte aligned");
-    launch_chained(dequant_bf16_kernel, dim3((unsigned)((OUT + 255) / 256), (unsigned)(K / BLOCK)), dim3(256), 0,
-                   static_cast<cudaStream_t>(stream), scale_exp, upper_cm, shared_cm, static_cast<__nv_bfloat16*>(Wbf), OUT, f);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (u == 4) launch_dequant_gs<4>(scale_exp, upper_cm, shared_cm, Wbf, OUT, K / BLOCK, f.lg_gs, st);
+    else if (u == 3) launch_dequant_gs<3>(scale_exp, upper_cm, shared_cm, Wbf, OUT, K / BLOCK, f.lg_gs, st);
+    else launch_dequant_gs<2>(scale_exp, upper_cm, shared_cm, Wbf, OUT, K / BLOCK, f.lg_gs, st);
     count_launch();
     return check_launch("dequant_bf16");
 }
