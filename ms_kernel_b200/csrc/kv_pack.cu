@@ -11,6 +11,12 @@
 #include "sm100_ptx.cuh"
 
 namespace msaq {
+
+// the packer of the gs = 2 formats, weight_pack.cu
+bool weight_pack_usable(const void* W, const void* upper_cm, const void* shared_cm, int64_t OUT, int64_t nb, int gs);
+int weight_pack_gs2(const void* W, int w_is_bf16, int8_t* scale_exp, uint8_t* upper, uint8_t* shared, uint8_t* upper_cm,
+                    uint8_t* shared_cm, int64_t OUT, int64_t nb, int u, cudaStream_t st);
+
 namespace {
 
 constexpr int ROWS_PER_CTA = 4;   // warps per block, one row each
@@ -283,6 +289,8 @@ extern "C" int msaq_pack_weight(const void* W, int w_is_bf16, int8_t* scale_exp,
     if (!W) return fail(MSAQ_ERR_ARG, "W is null");
     if (OUT <= 0 || K <= 0 || K % BLOCK) return fail(MSAQ_ERR_ARG, "K must be a positive multiple of 32");
     const int64_t nb = K / BLOCK, total = OUT * nb;
+    if (weight_pack_usable(W, upper_cm, shared_cm, OUT, nb, gs))
+        return weight_pack_gs2(W, w_is_bf16, scale_exp, upper, shared, upper_cm, shared_cm, OUT, nb, u, static_cast<cudaStream_t>(stream));
     launch_chained(pack_weight_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, static_cast<cudaStream_t>(stream), W, w_is_bf16, scale_exp, upper, shared, upper_cm, shared_cm, OUT, nb, f);
     count_launch();
     return check_launch("pack_weight");
