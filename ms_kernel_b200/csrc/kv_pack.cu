@@ -60,6 +60,50 @@ quantize_rows_kernel(const QuantJobs jobs, RowMap map, Fmt f) {
     quantize_row_warp<EPL>(job, map.rope, row, head, key, map.Lcap, f, rowbuf[warp], &codes[warp][0][0], lane);
 }
 
+// The gs = 2 formats: eight values per lane, 8 / EPL rows per warp.  Bound by HBM for a prompt (356 bytes per row of 128).
+// One warp per row with a lane per element of one block after another (quantize_rows_kernel, still the kernel of the
+// other group sizes and of MXINT8) spends its time on float64, shared-memory atomics and the four dependent blocks:
+// a prefill of 8 heads x 8191 keys, K and V one after the other, 155 -> 30 us.
+template <int EPL, int U>
+__global__ void __launch_bounds__(ROWS_PER_CTA * 32)
+quantize_rows8_kernel(const QuantJobs jobs, RowMap map) {
+    chain_release();
+    chain_wait();
+    constexpr int ROWS = 8 / EPL, LANES = 4 * EPL;
+    const QuantJob job = blockIdx.y == 0 ? jobs.j[0] : jobs.j[1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t row = ((int64_t)blockIdx.x * ROWS_PER_CTA + warp) * ROWS + lane / LANES;
+    bool live = row < map.rows;
+    int64_t head = row, key = map.key0;
+    if (map.rows_per_head > 1) {
+        if (map.rows <= UINT32_MAX) {                         // a 64-bit division costs more than the rest of the addressing
+            const uint32_t h = (uint32_t)row / (uint32_t)map.rows_per_head;
+            head = h;
+            key += (uint32_t)row - h * (uint32_t)map.rows_per_head;
+        } else {
+            head = row / map.rows_per_head;
+            key += row % map.rows_per_head;
+        }
+    }
+    if (map.pos && live) {                                    // range check: see quantize_rows_kernel
+        key = map.pos[head / map.heads_per_seq];
+        if (key < 0 || key >= map.Lcap) {
+            if (lane % LANES == 0 && map.sticky) atomicOr(map.sticky, BAD_APPEND_POS);
+            live = false;
+        }
+    }
+    quantize_rows8_warp<EPL, U>(job, map.rope, row, head, key, map.Lcap, live, lane);
+}
+
+template <int EPL>
+void launch_rows8(const QuantJobs& jobs, int n_jobs, const RowMap& map, int u, cudaStream_t st) {
+    constexpr int ROWS = ROWS_PER_CTA * (8 / EPL);
+    const dim3 grid((unsigned)((map.rows + ROWS - 1) / ROWS), (unsigned)n_jobs), block(ROWS_PER_CTA * 32);
+    if (u == 4) launch_chained(quantize_rows8_kernel<EPL, 4>, grid, block, 0, st, jobs, map);
+    else if (u == 3) launch_chained(quantize_rows8_kernel<EPL, 3>, grid, block, 0, st, jobs, map);
+    else launch_chained(quantize_rows8_kernel<EPL, 2>, grid, block, 0, st, jobs, map);
+}
+
 template <int EPL>
 __global__ void __launch_bounds__(ROWS_PER_CTA * 32)
 hadamard_rotate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, int64_t N) {
@@ -151,6 +195,18 @@ pack_weight_kernel(const void* __restrict__ W, int w_is_bf16, int8_t* __restrict
 
 int launch_rows(const QuantJobs& jobs, int n_jobs, const RowMap& map, int64_t D, const Fmt& f, cudaStream_t st) {
     if (map.rows == 0) return MSAQ_OK;
+    bool rows8 = f.gs == 2;                                   // 16-byte reads, word and half-word stores
+    for (int i = 0; i < n_jobs; ++i)
+        rows8 = rows8 && !jobs.j[i].mx && !(reinterpret_cast<uintptr_t>(jobs.j[i].X) & 15) &&
+                !(reinterpret_cast<uintptr_t>(jobs.j[i].upper) & 3) && !(reinterpret_cast<uintptr_t>(jobs.j[i].shared) & 1);
+    if (rows8 && (D == 32 || D == 64 || D == 128 || D == 256)) {
+        if (D == 32) launch_rows8<1>(jobs, n_jobs, map, f.u, st);
+        else if (D == 64) launch_rows8<2>(jobs, n_jobs, map, f.u, st);
+        else if (D == 128) launch_rows8<4>(jobs, n_jobs, map, f.u, st);
+        else launch_rows8<8>(jobs, n_jobs, map, f.u, st);
+        count_launch();
+        return check_launch("quantize_rows8");
+    }
     const dim3 grid((unsigned)((map.rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), (unsigned)n_jobs);
     const dim3 block(ROWS_PER_CTA * 32);
     switch (D) {

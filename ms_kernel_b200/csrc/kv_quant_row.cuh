@@ -5,6 +5,7 @@
 #pragma once
 
 #include "msaq_common.cuh"
+#include "quant8.cuh"
 #include "sm100_ptx.cuh"
 
 namespace msaq {
@@ -112,6 +113,51 @@ __device__ __forceinline__ void quantize_row_warp(const QuantJob& job, const Rop
         if (lane < f.SB) job.shared[slot * f.SB + lane] = (uint8_t)(cw[7 + (lane >> 2)] >> ((lane & 3) * 8));
         if (lane == 0) job.scale_exp[slot] = (int8_t)e;
     }
+}
+
+// The same for the gs = 2 formats with eight consecutive values per lane (quant8.cuh): a warp takes 8 / EPL rows at once,
+// 4 * EPL lanes to a row, and nothing goes through shared memory.  `row`, `head`, `key` and `live` are the lane's row's;
+// lanes of a row that is not live load and store nothing.  job.X must be 16-byte aligned, job.upper 4-, job.shared 2-byte.
+template <int EPL, int U>
+__device__ __forceinline__ void quantize_rows8_warp(const QuantJob& job, const Rope& rope, int64_t row, int64_t head, int64_t key,
+                                                    int64_t Lcap, bool live, int lane) {
+    constexpr int D = 32 * EPL, NB = EPL, LANES = 4 * EPL, UB = 4 * (8 - U), SB = 2 * U;
+    const int l = lane % LANES;
+    float v[8];
+    const uint4 raw = live ? *reinterpret_cast<const uint4*>(job.X + row * D + l * 8) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = bf16_lo(w[i]); v[2 * i + 1] = bf16_hi(w[i]); }
+    if (job.rope && rope.cos && live) {
+        const int64_t at = (rope.rows == 1 ? 0 : key) * (D / 2) + l * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rope_pair(v[2 * i], v[2 * i + 1], rope.cos[at + i], rope.sin[at + i], &v[2 * i], &v[2 * i + 1]);
+    }
+    if (job.rot != 0) {                                       // the butterfly of fwht_warp, eight values per lane
+#pragma unroll
+        for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if ((i & h) == 0) {
+                    const float a = v[i], b = v[i + h];
+                    v[i] = a + b;
+                    v[i + h] = a - b;
+                }
+#pragma unroll
+        for (int m = 1; m < LANES; m <<= 1)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float other = __shfl_xor_sync(0xffffffffu, v[i], m);
+                v[i] = (lane & m) ? (other - v[i]) : (v[i] + other);
+            }
+        const float inv = (float)(1.0 / sqrt((double)D));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= inv;
+    }
+    const Codes8 c = quant8<U>(v);
+    const int64_t slot = (head * NB + (l >> 2)) * Lcap + key;
+    quant8_store<U>(c, lane, live, job.upper + slot * UB, job.shared + slot * SB);
+    if (live && (lane & 3) == 0) job.scale_exp[slot] = (int8_t)c.e;
 }
 
 }  // namespace msaq
