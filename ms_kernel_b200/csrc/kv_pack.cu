@@ -63,7 +63,7 @@ quantize_rows_kernel(const QuantJobs jobs, RowMap map, Fmt f) {
 // The gs = 2 formats: eight values per lane, 8 / EPL rows per warp.  Bound by HBM for a prompt (356 bytes per row of 128).
 // One warp per row with a lane per element of one block after another (quantize_rows_kernel, still the kernel of the
 // other group sizes and of MXINT8) spends its time on float64, shared-memory atomics and the four dependent blocks:
-// a prefill of 8 heads x 8191 keys, K and V one after the other, 155 -> 30 us.
+// a prefill of 8 heads x 8191 keys, K and V one after the other, 155 -> 27 us.
 template <int EPL, int U>
 __global__ void __launch_bounds__(ROWS_PER_CTA * 32)
 quantize_rows8_kernel(const QuantJobs jobs, RowMap map) {

@@ -4,7 +4,7 @@
 // blocks; four lanes share a 32-block (quant8.cuh), so a warp reads 64-byte runs and writes the column-major planes as
 // they come; the bytes of the row-major planes go through shared memory and leave as 128-byte rows.  One thread per
 // 32-block with byte stores (kv_pack.cu, still the packer of the other group sizes) reads 64 bytes per lane a row apart
-// and scatters single bytes: 14336 x 4096 bf16 to u = 4, 485 -> 86 us.
+// and scatters single bytes: 14336 x 4096 bf16 to u = 4, 485 -> 72 us.
 // Behaviour: ms_lib/pack.py:101-137 of the reference (`pack_weight`).
 #include "quant8.cuh"
 #include "sm100_ptx.cuh"
