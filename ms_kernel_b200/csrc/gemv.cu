@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "gemv_mma.cuh"
+#include "gemv_direct.cuh"
 #include "gemv_reg.cuh"
 #include "gemv_umma.cuh"
 
@@ -227,6 +228,13 @@ struct RegPlan {
     size_t partial_off, total;
 };
 
+// Whether the register kernel is the one for these sizes (where the direct kernels are not).  u = 4 from five to eight rows:
+// up to about 100 MB (8192x8192, eight rows: 31.3 us on the integer kernel, 24.6; 28672x4096: 36.4, 35.9; 57344x8192, 367 MB:
+// 95.4, 110.4).
+bool reg_serves(int64_t M, int64_t OUT, int64_t NB, int u) {
+    return M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M || (M >= 5 && OUT * NB * 25 <= (100LL << 20)));
+}
+
 RegPlan plan_reg(int64_t M, int64_t OUT, int64_t NB, int u) {
     RegPlan p;
     GemvSchedule& s = p.sch;
@@ -290,9 +298,40 @@ int launch_xprep(const XprepArgs& xa, int mode, unsigned grid, cudaStream_t st) 
     return check_launch("gemv_xprep");
 }
 
+// ---- no partial sums in global memory: matrices of one wave (gemv_direct_pick), up to a size -------
+// The limits are where the pipelined kernels overtake (us per call, pipelined -> direct):
+//   u4, 1-2 rows   4096x4096 10.5 -> 6.8   8192x8192 19.3 -> 14.4   4096x28672 (92 MB) 30.0 -> 24.4   1024x8192 14.4 -> 5.8
+//   u4, 3-4 rows   4096x4096 12.1 -> 7.8   8192x8192 25.2 -> 20.0   8192x14336 (92 MB) 33.1 -> 32.3, 4096x28672 31.7 -> 33.8
+//   u4, 5-8 rows   4096x4096 16.7 -> 7.9   8192x8192 31.0 -> 22.0   4096x28672 38.3 -> 37.8
+//   u4, 9-16 rows  4096x4096 13.9 -> 8.5   4096x14336 (46 MB) 25.8 -> 22.0   8192x8192 (52 MB) 25.7 -> 26.7
+//   u3             4096x4096 14.1 -> 8.8   4096x14336, 8 rows 26.9 -> 22.8, 16 rows 28.8 -> 30.7
+//   u2             4096x4096 13.6 -> 8.0   4096x14336 (53 MB), 8 rows 25.6 -> 21.5, 16 rows 27.6 -> 23.4
+// The test hook stops a copy-issuing thread: it belongs to the pipelined kernels, which run while it is set.
+bool direct_usable(const void* X, int mode, int64_t M, int64_t OUT, int64_t NB, int u) {
+    if (M > (mode == XP_PLAIN ? GD_MAX_M : 4) || option_test_skip_stage() >= 0 || (reinterpret_cast<uintptr_t>(X) & 15)) return false;
+    const int64_t limit = u == 4 ? (M <= 2 ? 100 : M <= 8 ? 60 : 48) : u == 2 || M <= 8 ? 60 : 24;
+    int cg, cs;
+    return OUT * NB * (gr_ub(u) + gr_sb(u) + 1) <= (limit << 20) && gemv_direct_pick(M, OUT, NB, u, &cg, &cs);
+}
+
+int run_direct(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y,
+               float* Yf, int64_t M, int64_t OUT, int64_t NB, int u, const PeerPush* push, const void* res, cudaStream_t st) {
+    const int64_t K = NB * BLOCK;
+    int cg = 1, cs = 1;
+    gemv_direct_pick(M, OUT, NB, u, &cg, &cs);
+    GemvDirectArgs a{se, up, sh, X, pro.r, static_cast<__nv_bfloat16*>(pro.h_out), static_cast<__nv_bfloat16*>(Y), Yf,
+                     static_cast<const __nv_bfloat16*>(res), (int)M, (int)OUT, (int)NB,
+                     (int)(pro.mode == XP_SILU_MUL ? 2 * K : K), pro.r_is_f32, option_early_weights() ? 1 : 0, cs, pro.eps,
+                     push ? *push : PeerPush{}};
+    return gemv_direct_launch(a, u, pro.mode, cg, st);
+}
+
 int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh,
             void* Y, float* Yf, int64_t M, int64_t OUT, int64_t NB, void* ws, cudaStream_t st, int fmt = GF_MSAQ_U4,
             const PeerPush* push = nullptr, const void* res = nullptr) {
+    // (five rows and more without a prologue: as gemv_dispatch chooses, so that a residual add or a push changes no bit)
+    if (fmt == GF_MSAQ_U4 && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4))
+        return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, push, res, st);
     const MmaPlan p = plan_mma(M, OUT, NB, fmt);
     uint8_t* base = static_cast<uint8_t*>(ws);
     int* status = reinterpret_cast<int*>(base);
@@ -392,8 +431,10 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     // the tensor-memory epilogue stores 16 outputs at a time: Y (and Y_f32) must be 16-byte aligned for it
     const bool tm_ok = aligned && umma_eligible(OUT, u, gs, cm) && option_tensor_memory() &&
                        !((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15);
+    if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u))
+        return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, nullptr, nullptr, st);
     // up to 32 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
-    if (tm_ok && M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
+    if (tm_ok && reg_serves(M, OUT, NB, u) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
         const RegPlan p = plan_reg(M, OUT, NB, u);
         if (ws_bytes >= p.total) return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, p, ws, st);
     }
@@ -433,7 +474,7 @@ size_t msaq::gemv_workspace_front(int64_t M, int64_t OUT, int64_t NB, int u, int
 
 extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
     size_t bytes = gemv_workspace_min(M, OUT, NB, u, gs);
-    if (bytes && umma_eligible(OUT, u, gs, true) && M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M)) {
+    if (bytes && umma_eligible(OUT, u, gs, true) && reg_serves(M, OUT, NB, u)) {
         const size_t reg = plan_reg(M, OUT, NB, u).total;
         if (reg > bytes) bytes = reg;
     }
@@ -542,7 +583,10 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
     const bool ok = !((reinterpret_cast<uintptr_t>(x) & 15) | (reinterpret_cast<uintptr_t>(y) & 7) |
                       (reinterpret_cast<uintptr_t>(residual) & 7)) && M < GU_MIN_M &&
-                    mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true);
+                    mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true) &&
+                    // sizes whose plain GEMV is the register kernel's take its sum and add behind it
+                    !(prologue == MSAQ_PRO_NONE && M > 4 && option_tensor_memory() && reg_serves(M, OUT, NB, u) &&
+                      !direct_usable(x, XP_PLAIN, M, OUT, NB, u));
     if (ok) {
         const Prologue pro{prologue, nullptr, 0, nullptr, eps};
         return run_mma(static_cast<const __nv_bfloat16*>(x), pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB,

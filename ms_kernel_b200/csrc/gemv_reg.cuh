@@ -80,7 +80,6 @@ __device__ __forceinline__ GrLane gr_lane(int t) {
 // q = up * 2^u + sh.  A code with its sign bit flipped, dropped into the mantissa of bf16 128.0, reads as 128 + 2^(b-1) + code
 // (b its width).  h = sh * 2^e and then h + up * 2^(u+e) are formed with one fused multiply-add each; every value on the
 // way is an integer of at most eight significant bits times a power of two, so nothing is rounded.
-// ub, sb, eb: shared-memory addresses of this lane's codes and of the row's scale; OFF*: constant distances to this row.
 // The constants of the decode below, read back from shared memory once: as literals they are put into registers again at
 // every use (LOP3 and HFMA2 take one immediate at most), which doubles the instructions of a step.
 template <int U>
@@ -108,20 +107,23 @@ struct GrConst {
     }
 };
 
-template <int U, int OFFU, int OFFS, int OFFE>
-__device__ __forceinline__ void gr_decode_row(uint32_t ub, uint32_t sb, uint32_t eb, const GrLane& ln, const GrConst<U>& k,
-                                              uint32_t (&w)[4]) {
+// A lane's share of a row's packed block as loaded: u = 4: w0, s0; u = 3: both words and both half-words; u = 2: both words, s0.
+struct GrRaw {
+    uint32_t w0, w1, s0, s1;
+    int e;
+};
+
+template <int U>
+__device__ __forceinline__ void gr_decode(const GrRaw& in, const GrLane& ln, const GrConst<U>& k, uint32_t (&w)[4]) {
     constexpr int WB = 8 - U;
-    const uint32_t s = (uint32_t)(lds_s8<OFFE>(eb) * 0x00800080 + 0x3F803F80);        // 2^e twice
+    const uint32_t s = (uint32_t)(in.e * 0x00800080 + 0x3F803F80);                    // 2^e twice
     const uint32_t su = hfma2_bf16(s, k.two_u, k.neg0), ns = hfma2_bf16(s, k.soff, k.neg0);
 
     uint32_t f[4];                       // upper codes j (low half) and j + 4 (high half), other bits arbitrary
     if constexpr (U == 4) {
-        const uint32_t v = lds32<OFFU>(ub);
-        f[0] = v; f[1] = v >> 4; f[2] = v >> 8; f[3] = v >> 12;
+        f[0] = in.w0; f[1] = in.w0 >> 4; f[2] = in.w0 >> 8; f[3] = in.w0 >> 12;
     } else {
-        const uint32_t w0 = lds32<OFFU>(ub), w1 = lds32<OFFU + 4>(ub);
-        const uint32_t lo = __funnelshift_r(w0, w1, ln.up_shift), hi = w1 >> ln.up_shift;   // bits 0..31, 32.. of this lane's run
+        const uint32_t lo = __funnelshift_r(in.w0, in.w1, ln.up_shift), hi = in.w1 >> ln.up_shift;  // bits 0..31, 32.. of this lane's run
         const uint32_t up4 = __funnelshift_r(lo, hi, 4 * WB);                               // codes 4..7
         const uint32_t c = prmt(lo, up4, 0x5410u);                                          // low halves
         f[0] = c;
@@ -136,18 +138,30 @@ __device__ __forceinline__ void gr_decode_row(uint32_t ub, uint32_t sb, uint32_t
         }
     }
     uint32_t g;                          // shared codes 0, 1 (low half) and 2, 3 (high half)
-    if constexpr (U == 4) g = prmt(lds_u16<OFFS>(sb), 0u, 0x4140u);
+    if constexpr (U == 4) g = prmt(in.s0, 0u, 0x4140u);
     else if constexpr (U == 3) {
-        const uint32_t v = prmt(lds_u16<OFFS>(sb), lds_u16<OFFS>(sb - ln.sh_off + ln.sh_off2), 0x5410u) >> ln.sh_shift & 0xFFFu;
+        const uint32_t v = prmt(in.s0, in.s1, 0x5410u) >> ln.sh_shift & 0xFFFu;
         g = v | (v << 10);
-    } else {
-        uint32_t v;
-        asm volatile("ld.shared.u8 %0, [%1+%2];" : "=r"(v) : "r"(sb), "n"(OFFS));
-        g = v | (v << 12);
-    }
+    } else g = in.s0 | (in.s0 << 12);
     const uint32_t h0 = hfma2_bf16(and_xor(g, k.sm, k.sx), s, ns), h1 = hfma2_bf16(and_xor(g >> U, k.sm, k.sx), s, ns);
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[j] = hfma2_bf16(hfma2_bf16(and_xor(f[j], k.um, k.ux), k.one, k.uoff), su, j < 2 ? h0 : h1);
+}
+
+// The same from shared memory: ub, sb, eb are the addresses of this lane's codes and of the row's scale, OFF* constant
+// distances from there.
+template <int U, int OFFU, int OFFS, int OFFE>
+__device__ __forceinline__ void gr_decode_row(uint32_t ub, uint32_t sb, uint32_t eb, const GrLane& ln, const GrConst<U>& k,
+                                              uint32_t (&w)[4]) {
+    GrRaw r;
+    r.e = lds_s8<OFFE>(eb);
+    r.w0 = lds32<OFFU>(ub);
+    r.w1 = U == 4 ? 0u : lds32<OFFU + 4>(ub);
+    r.s1 = 0u;
+    if constexpr (U == 2) asm volatile("ld.shared.u8 %0, [%1+%2];" : "=r"(r.s0) : "r"(sb), "n"(OFFS));
+    else r.s0 = lds_u16<OFFS>(sb);
+    if constexpr (U == 3) r.s1 = lds_u16<OFFS>(sb - ln.sh_off + ln.sh_off2);
+    gr_decode<U>(r, ln, k, w);
 }
 
 // K block J of a stage: its activation fragments, then group Q = 0.. of the warp's columns.

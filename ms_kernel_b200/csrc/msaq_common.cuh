@@ -71,20 +71,36 @@ int* sticky_status();         // device address of the per-device status word on
 // block exits; with it 0.9 us after the staging kernel starts).
 void prefer_max_shared(const void* kernel);      // once per (kernel, device), only while the option is on
 
+// The same in clusters of `cluster` thread blocks (1: none).
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, cudaStream_t st,
+                                          A&&... args) {
     prefer_max_shared(reinterpret_cast<const void*>(kernel));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (option_chained_launch()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = option_chained_launch() ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_chained_cluster(kernel, grid, block, smem, 1, st, std::forward<A>(args)...);
 }
 
 // Rotary position embedding tables as the reference's harness builds them (tests/harness_batchsweep.py:

@@ -1,0 +1,99 @@
+"""GPU parity of the GEMVs without partial sums in global memory (csrc/gemv_direct.cuh) at the sizes where they can go wrong:
+one 32-block, fewer blocks than warps, odd counts, ragged column tiles of every width, clusters (few columns, long K), the
+edges of the row counts -- against the float64 oracle, and fused prologues, residual add and fp32 output against the
+separate steps."""
+
+import numpy as np
+import pytest
+import torch
+
+from conftest import F32_REL_FRO_TOL, MAX_ABS_REL_TOL, REL_FRO_TOL
+from oracle import msaq_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("u", (2, 3, 4))
+@pytest.mark.parametrize("M", (1, 2, 3, 4, 5, 8, 9, 16))
+@pytest.mark.parametrize("OUT,K", [(16, 32), (48, 480), (1040, 544), (304, 8224), (4752, 96), (7120, 64)])
+def test_edges(rng, u, M, OUT, K):
+    import cabi
+    W = orc.to_bf16((rng.standard_normal((OUT, K)) * rng.uniform(0.005, 0.08, (OUT, 1))).astype(np.float32))
+    X = orc.to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    p = orc.pack_weight(W, u, 2)
+    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    cabi.check_output(got, gotf, orc.wonly_matmul(p, X), MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+
+
+@pytest.mark.parametrize("M", (1, 2, 4))
+@pytest.mark.parametrize("OUT,K", [(1024, 8192), (4096, 4096), (4800, 512), (80, 96)])
+def test_fused_prologues(rng, M, OUT, K):
+    """The prologue's values are those of the separate kernels (the row norm to a rounding: its sum runs in another order)."""
+    from ms_kernel_b200 import ops, pack
+    msaq = torch.ops.msaq
+    W = (torch.randn((OUT, K), device="cuda") * 0.02).to(torch.bfloat16)
+    lin = ops.PackedLinear(pack.pack_weight(W, 4, 2), "cuda")
+    h = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    gu = torch.randn((M, 2 * K), device="cuda").to(torch.bfloat16)
+    res = torch.randn((M, OUT), device="cuda").to(torch.bfloat16)
+    plain = lin.fwd(msaq.silu_mul(gu)).reshape(M, OUT)
+    assert torch.equal(lin.fwd_fused(gu, ops.PRO_SILU_MUL), plain)
+    assert torch.equal(lin.fwd_fused(gu, ops.PRO_SILU_MUL, out_f32=True).to(torch.bfloat16), plain)
+    assert torch.equal(lin.fwd_fused_add(gu, ops.PRO_SILU_MUL, res), msaq.add_residual(res, plain.contiguous()))
+    want = lin.fwd(msaq.rmsnorm(h, 1e-5)).reshape(M, OUT).float().cpu().numpy()
+    assert orc.rel_fro(lin.fwd_fused(h, ops.PRO_RMSNORM).float().cpu().numpy(), want) < REL_FRO_TOL
+    for delta in (torch.randn((M, K), device="cuda"), torch.randn((M, K), device="cuda").to(torch.bfloat16)):
+        hn = msaq.add_residual(h, delta)
+        want = lin.fwd(msaq.rmsnorm(hn, 1e-5)).reshape(M, OUT).float().cpu().numpy()
+        got, hn2 = lin.fwd_fused(h, ops.PRO_ADD_RMSNORM, delta)
+        assert torch.equal(hn2, hn)
+        assert orc.rel_fro(got.float().cpu().numpy(), want) < REL_FRO_TOL
+
+
+@pytest.mark.parametrize("M", (5, 8))
+@pytest.mark.parametrize("OUT,K", [(512, 1024), (10240, 1024)])
+def test_residual_add_of_five_to_eight_rows(rng, M, OUT, K):
+    """Without a prologue the sum is the plain GEMV's, whichever kernel that is."""
+    from ms_kernel_b200 import ops, pack
+    W = (torch.randn((OUT, K), device="cuda") * 0.02).to(torch.bfloat16)
+    lin = ops.PackedLinear(pack.pack_weight(W, 4, 2), "cuda")
+    x = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    res = torch.randn((M, OUT), device="cuda").to(torch.bfloat16)
+    assert torch.equal(lin.fwd_fused_add(x, ops.PRO_NONE, res), torch.ops.msaq.add_residual(res, lin.fwd(x)))
+
+
+@pytest.mark.parametrize("bad", (float("inf"), float("-inf"), float("nan")))
+@pytest.mark.parametrize("M", (1, 6))
+def test_non_finite_activation(rng, bad, M):
+    import cabi
+    OUT, K = 256, 8192
+    W = orc.to_bf16((rng.standard_normal((OUT, K)) * 0.02).astype(np.float32))
+    X = orc.to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    p = orc.pack_weight(W, 4, 2)
+    X[M - 1, K - 3] = bad
+    _, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    assert np.isnan(gotf[M - 1]).all() and np.isfinite(gotf[: M - 1]).all()
+
+
+def test_back_to_back_and_replayed(rng):
+    """Dependent launches in one stream and in a replayed graph: a cluster's shared memory is not left early."""
+    from ms_kernel_b200 import ops, pack
+    W = (torch.randn((1024, 1024), device="cuda") * 0.03).to(torch.bfloat16)
+    W2 = (torch.randn((1024, 8192), device="cuda") * 0.01).to(torch.bfloat16)
+    a, b = (ops.PackedLinear(pack.pack_weight(w, 4, 2), "cuda") for w in (W, W2))
+    x = torch.randn((1, 8192), device="cuda").to(torch.bfloat16)
+    step = lambda: a.fwd(a.fwd(b.fwd(x)))       # noqa: E731
+    want = step()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        step()
+    torch.cuda.current_stream().wait_stream(s)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = step()
+    for _ in range(20):
+        g.replay()
+        assert torch.equal(step(), want)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
