@@ -54,8 +54,8 @@ unsigned long long msaq_launch_count(void);
  *   tail of the kernel before it.  Results do not change: every kernel waits for its predecessor before it
  *   reads or writes anything another kernel produces or consumes.
  * MSAQ_OPT_TENSOR_MEMORY (default 1): batched GEMVs (u=4, gs=2, 9 rows and more) run on exact bf16 operands -- up to
- *   32 rows with warp-level MMAs on register operands, above on the tcgen05 tensor cores with accumulators in tensor
- *   memory; 0 keeps them on the warp-level integer MMA path (the paths agree to the output tolerance, not bit for bit).
+ *   64 rows with warp-level MMAs on register operands, above (and for large matrices from 33) on the tcgen05 tensor cores
+ *   with accumulators in tensor memory; 0 keeps them on the warp-level integer MMA path (the paths agree to the output tolerance, not bit for bit).
  * MSAQ_OPT_INKERNEL_STAGING (default 1): small integer-MMA GEMVs (up to four rows, no fused prologue, at most
  *   eighteen K blocks per thread block) convert their activations inside the main kernel, one launch per GEMV; 0
  *   runs the separate staging kernel in front, as all other launches do.  Same staged values either way.

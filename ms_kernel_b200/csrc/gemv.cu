@@ -215,7 +215,7 @@ int run_umma(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const 
     return MSAQ_OK;
 }
 
-// ---- register-operand path (gs = 2, column-major planes, OUT % 16 == 0, up to 32 rows) --------------
+// ---- register-operand path (gs = 2, column-major planes, OUT % 16 == 0, up to 64 rows) --------------
 // Against the tensor-memory kernel, which serves what is left, us per call (rows: 1 | 16 | 32):
 //   28672x4096 u3  53.9 | 57.3 | 61.7 -> 39.5 | 44.1 | 58.8     u4, 16 | 32 rows  52.2 | 56.9 -> 38.5 | 51.3
 //   4096x4096  u3  23.3 | 26.1 | 28.5 -> 13.9 | 15.5 | 19.8     u4                25.3 | 27.5 -> 14.4 | 18.5
@@ -229,20 +229,23 @@ struct RegPlan {
 };
 
 // Whether the register kernel is the one for these sizes (where the direct kernels are not).  u = 4 from five to eight rows:
-// up to about 100 MB (8192x8192, eight rows: 31.3 us on the integer kernel, 24.6; 28672x4096: 36.4, 35.9; 57344x8192, 367 MB:
-// 95.4, 110.4).
+// up to about 100 MB (8192x8192, eight rows: 31.3 us on the integer kernel, 24.6; 28672x4096: 36.4, 33.4; 57344x8192, 367 MB:
+// 95.4, 110.4).  From 33 rows on up to about 48 MB (64 rows against the tensor-memory kernel: 6144x4096 41.3 -> 25.6,
+// 4096x14336, 46 MB, 48.2 -> 44.5, 8192x8192, 52 MB, 46.8 -> 47.8, 28672x4096 67.9 -> 80.5).
 bool reg_serves(int64_t M, int64_t OUT, int64_t NB, int u) {
-    return M <= GR_MAX_M && (u != 4 || M >= GU_MIN_M || (M >= 5 && OUT * NB * 25 <= (100LL << 20)));
+    const int64_t bytes = OUT * NB * (gr_ub(u) + gr_sb(u) + 1);
+    if (M > GR_MAX_M || (M > 32 && bytes > (48LL << 20))) return false;
+    return u != 4 || M >= GU_MIN_M || (M >= 5 && bytes <= (100LL << 20));
 }
 
 RegPlan plan_reg(int64_t M, int64_t OUT, int64_t NB, int u) {
     RegPlan p;
     GemvSchedule& s = p.sch;
     const int64_t rows = M < GR_MAX_M ? M : GR_MAX_M;
-    p.mt = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
-    s.tc = GR_TC;
+    p.mt = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
+    s.tc = gr_tc(p.mt);
     s.nb = (int)((NB + GR_KB - 1) / GR_KB);
-    s.col_tiles = (int)((OUT + GR_TC - 1) / GR_TC);
+    s.col_tiles = (int)((OUT + s.tc - 1) / s.tc);
     const long long units = s.units(), slots = sm_count();
     s.grid = (int)(units < slots ? units : slots);
     s.max_slots = (int)(((long long)s.nb * s.grid + units - 1) / units) + 1;
@@ -433,7 +436,7 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
                        !((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15);
     if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u))
         return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, nullptr, nullptr, st);
-    // up to 32 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
+    // up to 64 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
     if (tm_ok && reg_serves(M, OUT, NB, u) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
         const RegPlan p = plan_reg(M, OUT, NB, u);
         if (ws_bytes >= p.total) return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, p, ws, st);

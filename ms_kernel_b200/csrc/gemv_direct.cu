@@ -43,18 +43,19 @@ bool integer(int64_t M, int u) { return u == 4 && M <= 4; }
 // columns, sixteen warps on four schedulers, `resident` thread blocks to an SM -- or a load's latency, and a cluster costs its
 // barriers.  So wide thread blocks in clusters win where the activations are expensive and K is long (4096 x 14336, one row,
 // us: one group 19.2, four groups and two thread blocks to a cluster 14.0), narrow ones without where it is short (2048 x
-// 2048: 3.5 against 4.9).  A cluster has to fit a GPC (some sixteen SMs of the eight can be counted on): clusters beyond that
-// wait for a second round (1216 x 18688, 19 clusters of seven: 14.6 us, 76 of three: 11.1 us).
+// 2048: 3.5 against 4.9).  Clusters that do not fit the GPCs wait for a second round (1216 x 18688,
+// 19 clusters of seven: 14.6 us, 76 of three: 11.1 us; the occupancy query counts 148, 74, 45, 33, 26, 22, 15 and 15 clusters of one
+// to eight thread blocks, one to an SM; GPCs differ by a few SMs from part to part, hence a little less here).
 bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs) {
     static const int int1[] = {1, 4, 0}, int4[] = {2, 4, 0}, bf4[] = {2, 3, 4, 0}, bf3[] = {2, 3, 0};
     const int* widths = integer(M, u) ? (M == 1 ? int1 : int4) : u == 4 ? bf4 : bf3;
     const int64_t stage = integer(M, u) ? 55 * M : 20, group = integer(M, u) ? 45 : (u == 4 ? 95 : u == 3 ? 115 : 105) + (M > 8 ? 15 : 0);
+    static const int fit[GD_MAX_CLUSTER + 1] = {0, 148, 74, 44, 32, 24, 20, 14, 14};
     int64_t best = INT64_MAX;
     for (const int* w = widths; *w; ++w) {
         const int64_t per_sm = integer(M, u) ? gd_int_per_sm(*w) : 1, tiles = (OUT + 16 * *w - 1) / (16 * *w);
         for (int n = 1; n <= GD_MAX_CLUSTER; ++n) {
-            const int64_t clusters = n == 1 ? sm_count() : n == 2 ? sm_count() / 2 : 8 * (16 / n);
-            if (tiles > clusters * per_sm) break;
+            if (tiles > (n == 1 ? sm_count() : fit[n]) * per_sm) break;
             if (n > 1 && NB < 2 * GD_WARPS * n) break;
             const int64_t resident = (tiles * n + sm_count() - 1) / sm_count(), iterations = (NB + GD_WARPS * n - 1) / (GD_WARPS * n);
             const int64_t issue = 4 * resident * (stage + *w * group) * 5 / 4;

@@ -406,11 +406,11 @@ gemv_direct_bf16_kernel(const GemvDirectArgs a) {
     __syncthreads();
     const GrConst<U> kc(smem_u32(consts));
 
-    float acc[CG][MT][4];
+    float acc[CG][gr_accs(MT)][4];
 #pragma unroll
     for (int q = 0; q < CG; ++q)
 #pragma unroll
-        for (int n = 0; n < MT; ++n) acc[q][n][0] = acc[q][n][1] = acc[q][n][2] = acc[q][n][3] = 0.0f;
+        for (int n = 0; n < gr_accs(MT); ++n) acc[q][n][0] = acc[q][n][1] = acc[q][n][2] = acc[q][n][3] = 0.0f;
     for (int kb0 = first; kb0 < a.NB; kb0 += 2 * stride) {
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
@@ -441,14 +441,16 @@ gemv_direct_bf16_kernel(const GemvDirectArgs a) {
                     uint32_t w0[4], w1[4];
                     gr_decode<U>(cur[d][q][0], ln, kc, w0);
                     gr_decode<U>(cur[d][q][1], ln, kc, w1);
-#pragma unroll
-                    for (int n = 0; n < MT; ++n) {
-                        mma_bf16_16816(acc[q][n], w0[0], w1[0], w0[1], w1[1], b[n][0], b[n][1]);
-                        mma_bf16_16816(acc[q][n], w0[2], w1[2], w0[3], w1[3], b[n][2], b[n][3]);
-                    }
+                    gr_mma<MT, gr_accs(MT)>(acc[q], w0, w1, b);
                 }
             }
         }
+    }
+    if constexpr (MT == 1) {
+#pragma unroll
+        for (int q = 0; q < CG; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[q][0][i] += acc[q][1][i];
     }
 #pragma unroll
     for (int half = 0; half < HALVES; ++half) {

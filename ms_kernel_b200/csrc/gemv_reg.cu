@@ -22,7 +22,7 @@ int launch_reg(const GemvRegArgs& a, cudaStream_t st) {
 
 template <int U>
 int launch_reg_mt(const GemvRegArgs& a, int mt, cudaStream_t st) {
-    return mt == 1 ? launch_reg<U, 1>(a, st) : mt == 2 ? launch_reg<U, 2>(a, st) : launch_reg<U, 4>(a, st);
+    return mt == 1 ? launch_reg<U, 1>(a, st) : mt == 2 ? launch_reg<U, 2>(a, st) : mt == 4 ? launch_reg<U, 4>(a, st) : launch_reg<U, 8>(a, st);
 }
 
 }  // namespace

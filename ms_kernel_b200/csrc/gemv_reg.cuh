@@ -1,8 +1,8 @@
-// Weight-only GEMV for small batches on register operands, Y[M][OUT] = X[M][K] * dequant(W)^T at gs = 2: the 5+3 and
-// 6+2 bit formats (u = 3, u = 2) up to 32 rows, and the nibble format (u = 4) from nine to 32.
+// Weight-only GEMV for small batches on register operands, Y[M][OUT] = X[M][K] * dequant(W)^T at gs = 2, up to 64 rows (which
+// sizes: reg_serves() in gemv.cu).
 //
-// What bounds it is the widening of the codes, then HBM.  The
-// tensor-memory kernel (gemv_umma.cuh) pays for the same widening a trip through shared memory, a proxy fence and two
+// What bounds it is the widening of the codes up to 16 rows, the rate of the warp-level MMA above (eight cycles each), then HBM.
+// The tensor-memory kernel (gemv_umma.cuh) pays for the same widening a trip through shared memory, a proxy fence and two
 // barrier hand-offs per unit with one thread block per SM, and its 128-row activation tile is mostly padding at these
 // batches.  Here a lane widens the codes of its own MMA fragment in registers and nothing else touches them:
 //   * the weights are the 16-row A operand of mma.m16n8k16 (bf16 in, fp32 out), eight activation rows the B operand;
@@ -25,9 +25,10 @@
 
 namespace msaq {
 
-constexpr int GR_MAX_M = 32;                       // activation rows per launch
-constexpr int GR_GROUPS = 2;                       // 128-column groups per tile
-constexpr int GR_TC = GR_GROUPS * GM_GROUP;        // 256 columns
+constexpr int GR_MAX_M = 64;                       // activation rows per launch
+// 128-column groups per tile, by n-tiles of eight activation rows: as many as the accumulators leave registers for
+__host__ __device__ constexpr int gr_groups_of(int mt) { return mt <= 4 ? 2 : 1; }
+__host__ __device__ constexpr int gr_tc(int mt) { return gr_groups_of(mt) * GM_GROUP; }
 constexpr int GR_KB = 4;                           // K blocks per ring stage
 // bytes between activation rows of a stage: 64 beyond the data, so that the 16-byte loads of two neighbouring rows fall
 // into different halves of the banks
@@ -38,10 +39,10 @@ __host__ __device__ constexpr int gr_sb(int u) { return 2 * u; }
 // with two teams has as many warps in flight as two thread blocks and leaves half the partial sums.
 constexpr int GR_TEAMS = 2;
 constexpr int GR_THREADS = GR_TEAMS * (GM_WARPS + 1) * 32;
-__host__ __device__ constexpr int gr_sub_bytes(int u) { return GR_TC * (gr_ub(u) + gr_sb(u) + 1); }    // one K block of a tile
-__host__ __device__ constexpr int gr_stage_bytes(int u, int mt) { return GR_KB * gr_sub_bytes(u) + mt * 8 * GR_XROW; }
+__host__ __device__ constexpr int gr_sub_bytes(int u, int mt) { return gr_tc(mt) * (gr_ub(u) + gr_sb(u) + 1); }    // one K block of a tile
+__host__ __device__ constexpr int gr_stage_bytes(int u, int mt) { return GR_KB * gr_sub_bytes(u, mt) + mt * 8 * GR_XROW; }
 // the accumulators that the other teams hand to the first
-__host__ __device__ constexpr int gr_merge_bytes(int mt) { return (GR_TEAMS - 1) * GM_WARPS * GR_GROUPS * mt * 512; }
+__host__ __device__ constexpr int gr_merge_bytes(int mt) { return (GR_TEAMS - 1) * GM_WARPS * gr_groups_of(mt) * mt * 512; }
 
 __device__ __forceinline__ uint32_t hfma2_bf16(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
@@ -164,48 +165,79 @@ __device__ __forceinline__ void gr_decode_row(uint32_t ub, uint32_t sb, uint32_t
     gr_decode<U>(r, ln, k, w);
 }
 
-// K block J of a stage: its activation fragments, then group Q = 0.. of the warp's columns.
-template <int U, int MT, int J, int Q, bool ALL>
-__device__ __forceinline__ void gr_groups(int nq, uint32_t ub, uint32_t sb, uint32_t eb, const GrLane& ln, const GrConst<U>& k,
-                                          const uint32_t (&b)[MT][4], float (&acc)[GR_GROUPS][MT][4]) {
-    if constexpr (Q < GR_GROUPS) {
-        if (ALL || Q < nq) {
-            constexpr int SUBJ = J * gr_sub_bytes(U), UB = gr_ub(U), SB = gr_sb(U);
-            constexpr int OU = SUBJ + Q * GM_GROUP * UB, OS = SUBJ + Q * GM_GROUP * SB, OE = SUBJ + Q * GM_GROUP;
-            uint32_t w0[4], w1[4];
-            gr_decode_row<U, OU, OS, OE>(ub, sb, eb, ln, k, w0);
-            gr_decode_row<U, OU + 8 * UB, OS + 8 * SB, OE + 8>(ub, sb, eb, ln, k, w1);
-#pragma unroll
-            for (int n = 0; n < MT; ++n) {
-                mma_bf16_16816(acc[Q][n], w0[0], w1[0], w0[1], w1[1], b[n][0], b[n][1]);
-                mma_bf16_16816(acc[Q][n], w0[2], w1[2], w0[3], w1[3], b[n][2], b[n][3]);
-            }
-        }
-        gr_groups<U, MT, J, Q + 1, ALL>(nq, ub, sb, eb, ln, k, b, acc);
-    }
+// K block J of a stage: its activation fragments and the weights of the warp's groups, in the order that leaves fewer registers
+// in use.  Every group is computed: columns beyond the matrix (a ragged last tile) come out as garbage that is not stored.
+template <int MT, int J, int N>
+__device__ __forceinline__ void gr_activation(uint32_t xb, uint32_t (&b)[4]) {
+    const uint4 x = lds128<N * 8 * GR_XROW + J * 64>(xb);
+    b[0] = prmt(x.x, x.z, 0x5410u);
+    b[1] = prmt(x.x, x.z, 0x7632u);
+    b[2] = prmt(x.y, x.w, 0x5410u);
+    b[3] = prmt(x.y, x.w, 0x7632u);
 }
 template <int MT, int J, int N>
 __device__ __forceinline__ void gr_activations(uint32_t xb, uint32_t (&b)[MT][4]) {
     if constexpr (N < MT) {
-        const uint4 x = lds128<N * 8 * GR_XROW + J * 64>(xb);
-        b[N][0] = prmt(x.x, x.z, 0x5410u);
-        b[N][1] = prmt(x.x, x.z, 0x7632u);
-        b[N][2] = prmt(x.y, x.w, 0x5410u);
-        b[N][3] = prmt(x.y, x.w, 0x7632u);
+        gr_activation<MT, J, N>(xb, b[N]);
         gr_activations<MT, J, N + 1>(xb, b);
     }
 }
+template <int U, int MT, int J, int Q>
+__device__ __forceinline__ void gr_weights(uint32_t ub, uint32_t sb, uint32_t eb, const GrLane& ln, const GrConst<U>& k,
+                                           uint32_t (&w0)[4], uint32_t (&w1)[4]) {
+    constexpr int SUBJ = J * gr_sub_bytes(U, MT), UB = gr_ub(U), SB = gr_sb(U);
+    constexpr int OU = SUBJ + Q * GM_GROUP * UB, OS = SUBJ + Q * GM_GROUP * SB, OE = SUBJ + Q * GM_GROUP;
+    gr_decode_row<U, OU, OS, OE>(ub, sb, eb, ln, k, w0);
+    gr_decode_row<U, OU + 8 * UB, OS + 8 * SB, OE + 8>(ub, sb, eb, ln, k, w1);
+}
+// The products of one group with N n-tiles: the first sixteen elements of the block against all of them, then the second, so
+// that no MMA waits for the one before it.  A single n-tile has two accumulators for that (added up at the end).
+__host__ __device__ constexpr int gr_accs(int mt) { return mt == 1 ? 2 : mt; }
+template <int N, int NACC>
+__device__ __forceinline__ void gr_mma(float (*acc)[4], const uint32_t (&w0)[4], const uint32_t (&w1)[4], const uint32_t (&b)[N][4]) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_bf16_16816(acc[n], w0[0], w1[0], w0[1], w1[1], b[n][0], b[n][1]);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mma_bf16_16816(acc[NACC > N ? n + 1 : n], w0[2], w1[2], w0[3], w1[3], b[n][2], b[n][3]);
+}
+template <int U, int MT, int J, int Q>
+__device__ __forceinline__ void gr_groups(uint32_t ub, uint32_t sb, uint32_t eb, const GrLane& ln, const GrConst<U>& k,
+                                          const uint32_t (&b)[MT][4], float (&acc)[gr_groups_of(MT)][gr_accs(MT)][4]) {
+    if constexpr (Q < gr_groups_of(MT)) {
+        uint32_t w0[4], w1[4];
+        gr_weights<U, MT, J, Q>(ub, sb, eb, ln, k, w0, w1);
+        gr_mma<MT, gr_accs(MT)>(acc[Q], w0, w1, b);
+        gr_groups<U, MT, J, Q + 1>(ub, sb, eb, ln, k, b, acc);
+    }
+}
+template <int MT, int J, int N>
+__device__ __forceinline__ void gr_rows(uint32_t xb, const uint32_t (&w0)[4], const uint32_t (&w1)[4], float (&acc)[MT][4]) {
+    if constexpr (N < MT) {                                                   // four n-tiles at a time
+        uint32_t b[4][4];
+        gr_activation<MT, J, N>(xb, b[0]);
+        gr_activation<MT, J, N + 1>(xb, b[1]);
+        gr_activation<MT, J, N + 2>(xb, b[2]);
+        gr_activation<MT, J, N + 3>(xb, b[3]);
+        gr_mma<4, 4>(&acc[N], w0, w1, b);
+        gr_rows<MT, J, N + 4>(xb, w0, w1, acc);
+    }
+}
 template <int U, int MT, int J>
-__device__ __forceinline__ void gr_blocks(int nblk, int nq, uint32_t ub, uint32_t sb, uint32_t eb, uint32_t xb, const GrLane& ln,
-                                          const GrConst<U>& k, float (&acc)[GR_GROUPS][MT][4]) {
+__device__ __forceinline__ void gr_blocks(int nblk, uint32_t ub, uint32_t sb, uint32_t eb, uint32_t xb, const GrLane& ln,
+                                          const GrConst<U>& k, float (&acc)[gr_groups_of(MT)][gr_accs(MT)][4]) {
     if constexpr (J < GR_KB) {
         if (J < nblk) {
-            uint32_t b[MT][4];
-            gr_activations<MT, J, 0>(xb, b);
-            if (nq >= GR_GROUPS) gr_groups<U, MT, J, 0, true>(nq, ub, sb, eb, ln, k, b, acc);
-            else gr_groups<U, MT, J, 0, false>(nq, ub, sb, eb, ln, k, b, acc);
+            if constexpr (gr_groups_of(MT) > 1) {
+                uint32_t b[MT][4];
+                gr_activations<MT, J, 0>(xb, b);
+                gr_groups<U, MT, J, 0>(ub, sb, eb, ln, k, b, acc);
+            } else {
+                uint32_t w0[4], w1[4];
+                gr_weights<U, MT, J, 0>(ub, sb, eb, ln, k, w0, w1);
+                gr_rows<MT, J, 0>(xb, w0, w1, acc[0]);
+            }
         }
-        gr_blocks<U, MT, J + 1>(nblk, nq, ub, sb, eb, xb, ln, k, acc);
+        gr_blocks<U, MT, J + 1>(nblk, ub, sb, eb, xb, ln, k, acc);
     }
 }
 
@@ -239,8 +271,8 @@ gemv_reg_kernel(const GemvRegArgs a) {
     __shared__ unsigned int marker_sh[GM_WARPS];
     __shared__ uint32_t consts[GrConst<U>::N];
 
-    constexpr int UB = gr_ub(U), SB = gr_sb(U);
-    constexpr int OFF_SH = GR_TC * UB, OFF_SC = GR_TC * (UB + SB), SUB = gr_sub_bytes(U), OFF_X = GR_KB * SUB;
+    constexpr int UB = gr_ub(U), SB = gr_sb(U), GR_GROUPS = gr_groups_of(MT), GR_TC = gr_tc(MT);
+    constexpr int OFF_SH = GR_TC * UB, OFF_SC = GR_TC * (UB + SB), SUB = gr_sub_bytes(U, MT), OFF_X = GR_KB * SUB;
     constexpr int STAGE = gr_stage_bytes(U, MT);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -319,11 +351,11 @@ gemv_reg_kernel(const GemvRegArgs a) {
     const GrConst<U> kc(smem_u32(consts));
     const uint32_t aU = smem0 + r0 * UB + ln.up_off, aS = smem0 + OFF_SH + r0 * SB + ln.sh_off, aE = smem0 + OFF_SC + r0;
     const uint32_t aX = smem0 + OFF_X + g * GR_XROW + t * 16;
-    float acc[GR_GROUPS][MT][4];
+    float acc[GR_GROUPS][gr_accs(MT)][4];
 #pragma unroll
     for (int q = 0; q < GR_GROUPS; ++q)
 #pragma unroll
-        for (int n = 0; n < MT; ++n) acc[q][n][0] = acc[q][n][1] = acc[q][n][2] = acc[q][n][3] = 0.0f;
+        for (int n = 0; n < gr_accs(MT); ++n) acc[q][n][0] = acc[q][n][1] = acc[q][n][2] = acc[q][n][3] = 0.0f;
     bool aborted = false;
     int s = 0, seg = 0, next = team;                                         // ring stage and index of this team's next unit
     uint32_t ph = 0;
@@ -345,11 +377,20 @@ gemv_reg_kernel(const GemvRegArgs a) {
                 aborted = true;
             } else {
                 const uint32_t so = s * STAGE;
-                gr_blocks<U, MT, 0>(kleft, nq, aU + so, aS + so, aE + so, aX + so, ln, kc, acc);
+                gr_blocks<U, MT, 0>(kleft, aU + so, aS + so, aE + so, aX + so, ln, kc, acc);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_empty[s]));
             if (++s == sch.stages) { s = 0; ph ^= 1u; }
+        }
+        if constexpr (MT == 1) {
+#pragma unroll
+            for (int q = 0; q < GR_GROUPS; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[q][0][i] += acc[q][1][i];
+                    acc[q][1][i] = 0.0f;
+                }
         }
         {
             // the teams' sums come together: warp cw of each of the others hands its accumulators to warp cw of the first

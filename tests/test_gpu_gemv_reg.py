@@ -1,4 +1,4 @@
-"""GPU parity of the register-operand GEMV (csrc/gemv_reg.cuh: gs = 2, up to 32 rows) at the sizes where it can go wrong:
+"""GPU parity of the register-operand GEMV (csrc/gemv_reg.cuh: gs = 2, up to 64 rows) at the sizes where it can go wrong:
 one and a few K blocks (four to a ring stage, two teams), ragged tiles of 256 columns, the edges of the eight-row
 n-tiles, matrices that one thread block covers and matrices that many share -- against the float64 oracle."""
 
@@ -21,7 +21,8 @@ def _case(rng, OUT, K, u, M):
 
 @pytest.mark.parametrize("u", (2, 3, 4))
 @pytest.mark.parametrize("M,OUT,K", [(1, 16, 32), (8, 240, 96), (9, 256, 160), (16, 272, 4096), (17, 528, 288), (31, 16, 8224),
-                                     (32, 1040, 1312), (33, 256, 128)])
+                                     (32, 1040, 1312), (33, 256, 128),
+                                     (33, 144, 96), (61, 400, 8224), (64, 1040, 544), (65, 128, 64)])
 def test_edges(rng, u, M, OUT, K):
     import cabi
     X, p = _case(rng, OUT, K, u, M)
@@ -73,7 +74,7 @@ def test_bits_do_not_depend_on_the_workspace_contents(rng):
     assert np.array_equal(cabi.gemv("batched", x, pd, M=5)[1], first)
 
 
-@pytest.mark.parametrize("u,M", [(3, 2), (4, 12)])
+@pytest.mark.parametrize("u,M", [(3, 2), (4, 12), (4, 50)])
 def test_wait_gives_up_and_next_call_is_correct(rng, u, M):
     import cabi
     OUT, K = 2048, 2048
