@@ -35,6 +35,22 @@ int check_launch(const char* what) {
 }
 
 namespace {
+thread_local int tl_scopes = 0, tl_device = -1;       // entry points of this thread on the stack, and their device
+int ask_device() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess) return dev;
+    cudaGetLastError();
+    return -1;
+}
+}  // namespace
+
+DeviceScope::DeviceScope() {
+    if (tl_scopes++ == 0) tl_device = ask_device();
+}
+DeviceScope::~DeviceScope() { --tl_scopes; }
+int current_device() { return tl_scopes > 0 ? tl_device : ask_device(); }
+
+namespace {
 std::atomic<int> g_opt_chained{-1};
 std::atomic<int> g_opt_tmem{1};
 std::atomic<int> g_opt_polls{1 << 20};
@@ -73,10 +89,10 @@ int option_test_skip_stage() { return g_opt_skip.load(std::memory_order_relaxed)
 void prefer_max_shared(const void* kernel) {
     static std::mutex mu;
     static std::set<std::pair<const void*, int>> done;
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    std::lock_guard<std::mutex> lock(mu);
     if (!option_early_weights()) return;
+    const int dev = current_device();
+    if (dev < 0) return;
+    std::lock_guard<std::mutex> lock(mu);
     if (!done.insert({kernel, dev}).second) return;
     // a preference, not a requirement: a failure here changes nothing but the overlap
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
@@ -84,8 +100,8 @@ void prefer_max_shared(const void* kernel) {
 }
 
 int* sticky_status() {
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    const int dev = current_device();
+    if (dev < 0 || dev >= 64) return nullptr;
     int* p = g_sticky_ptr[dev].load(std::memory_order_acquire);
     if (!p) {
         void* q = nullptr;
@@ -121,8 +137,8 @@ std::atomic<int> g_sm[MAX_DEV];
 std::atomic<int> g_cc[MAX_DEV];
 
 int current_device_attr(std::atomic<int>* cache, cudaDeviceAttr attr) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return 0;
+    const int dev = current_device();
+    if (dev < 0 || dev >= MAX_DEV) return 0;
     int v = cache[dev].load(std::memory_order_relaxed);
     if (v == 0) {
         if (cudaDeviceGetAttribute(&v, attr, dev) != cudaSuccess) return 0;

@@ -84,8 +84,7 @@ template <int PASSES, int TC, int KB, bool INK, int FMT = GF_MSAQ_U4, bool PUSH 
 int launch_mma_ink(const GemvMmaArgs& a, cudaStream_t st) {
     static int configured[64] = {};                      // largest dynamic smem size set per device
     const int smem = a.sch.stages * KB * gm_stage_bytes(TC, PASSES, FMT) + a.table_bytes;
-    int dev = 0;
-    cudaGetDevice(&dev);
+    const int dev = current_device();
     if (dev >= 0 && dev < 64 && configured[dev] < smem) {
         if (cudaFuncSetAttribute(gemv_u4gs2_mma_kernel<PASSES, TC, KB, INK, FMT, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  smem) != cudaSuccess)
@@ -172,8 +171,7 @@ UmmaPlan plan_umma(int64_t M, int64_t OUT, int64_t NB, int u) {
 template <int U>
 int launch_umma(const GemvUmmaArgs& a, int smem, cudaStream_t st) {
     static int configured[64] = {};                      // largest dynamic smem size set per device
-    int dev = 0;
-    cudaGetDevice(&dev);
+    const int dev = current_device();
     if (dev >= 0 && dev < 64 && configured[dev] < smem) {
         if (cudaFuncSetAttribute(gemv_umma_kernel<U>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return fail(MSAQ_ERR_CUDA, "cannot reserve %d bytes of shared memory", smem);
@@ -310,18 +308,15 @@ int launch_xprep(const XprepArgs& xa, int mode, unsigned grid, cudaStream_t st) 
 //   u3             4096x4096 14.1 -> 8.8   4096x14336, 8 rows 26.9 -> 22.8, 16 rows 28.8 -> 30.7
 //   u2             4096x4096 13.6 -> 8.0   4096x14336 (53 MB), 8 rows 25.6 -> 21.5, 16 rows 27.6 -> 23.4
 // The test hook stops a copy-issuing thread: it belongs to the pipelined kernels, which run while it is set.
-bool direct_usable(const void* X, int mode, int64_t M, int64_t OUT, int64_t NB, int u) {
+bool direct_usable(const void* X, int mode, int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs) {
     if (M > (mode == XP_PLAIN ? GD_MAX_M : 4) || option_test_skip_stage() >= 0 || (reinterpret_cast<uintptr_t>(X) & 15)) return false;
     const int64_t limit = u == 4 ? (M <= 2 ? 100 : M <= 8 ? 60 : 48) : u == 2 || M <= 8 ? 60 : 24;
-    int cg, cs;
-    return OUT * NB * (gr_ub(u) + gr_sb(u) + 1) <= (limit << 20) && gemv_direct_pick(M, OUT, NB, u, &cg, &cs);
+    return OUT * NB * (gr_ub(u) + gr_sb(u) + 1) <= (limit << 20) && gemv_direct_pick(M, OUT, NB, u, cg, cs);
 }
 
 int run_direct(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y,
-               float* Yf, int64_t M, int64_t OUT, int64_t NB, int u, const PeerPush* push, const void* res, cudaStream_t st) {
+               float* Yf, int64_t M, int64_t OUT, int64_t NB, int u, int cg, int cs, const PeerPush* push, const void* res, cudaStream_t st) {
     const int64_t K = NB * BLOCK;
-    int cg = 1, cs = 1;
-    gemv_direct_pick(M, OUT, NB, u, &cg, &cs);
     GemvDirectArgs a{se, up, sh, X, pro.r, static_cast<__nv_bfloat16*>(pro.h_out), static_cast<__nv_bfloat16*>(Y), Yf,
                      static_cast<const __nv_bfloat16*>(res), (int)M, (int)OUT, (int)NB,
                      (int)(pro.mode == XP_SILU_MUL ? 2 * K : K), pro.r_is_f32, option_early_weights() ? 1 : 0, cs, pro.eps,
@@ -333,8 +328,9 @@ int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const
             void* Y, float* Yf, int64_t M, int64_t OUT, int64_t NB, void* ws, cudaStream_t st, int fmt = GF_MSAQ_U4,
             const PeerPush* push = nullptr, const void* res = nullptr) {
     // (five rows and more without a prologue: as gemv_dispatch chooses, so that a residual add or a push changes no bit)
-    if (fmt == GF_MSAQ_U4 && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4))
-        return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, push, res, st);
+    int cg = 1, cs = 1;
+    if (fmt == GF_MSAQ_U4 && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4, &cg, &cs))
+        return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, cg, cs, push, res, st);
     const MmaPlan p = plan_mma(M, OUT, NB, fmt);
     uint8_t* base = static_cast<uint8_t*>(ws);
     int* status = reinterpret_cast<int*>(base);
@@ -434,8 +430,9 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     // the tensor-memory epilogue stores 16 outputs at a time: Y (and Y_f32) must be 16-byte aligned for it
     const bool tm_ok = aligned && umma_eligible(OUT, u, gs, cm) && option_tensor_memory() &&
                        !((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15);
-    if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u))
-        return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, nullptr, nullptr, st);
+    int cg = 1, cs = 1;
+    if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u, &cg, &cs))
+        return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, cg, cs, nullptr, nullptr, st);
     // up to 64 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
     if (tm_ok && reg_serves(M, OUT, NB, u) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
         const RegPlan p = plan_reg(M, OUT, NB, u);
@@ -476,6 +473,7 @@ size_t msaq::gemv_workspace_front(int64_t M, int64_t OUT, int64_t NB, int u, int
 }
 
 extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
+    const DeviceScope device;
     size_t bytes = gemv_workspace_min(M, OUT, NB, u, gs);
     if (bytes && umma_eligible(OUT, u, gs, true) && reg_serves(M, OUT, NB, u)) {
         const size_t reg = plan_reg(M, OUT, NB, u).total;
@@ -487,6 +485,7 @@ extern "C" size_t msaq_wonly_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, 
 extern "C" int msaq_wonly_gemv(const void* x, const int8_t* scale_exp, const uint8_t* upper, const uint8_t* shared,
                                void* y, float* y_f32, int64_t OUT, int64_t NB, int u, int gs, void* workspace,
                                size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     return gemv_dispatch(x, scale_exp, upper, shared, y, y_f32, 1, OUT, NB, u, gs, false, workspace, workspace_bytes,
                          stream);
 }
@@ -494,6 +493,7 @@ extern "C" int msaq_wonly_gemv(const void* x, const int8_t* scale_exp, const uin
 extern "C" int msaq_wonly_gemv_wide(const void* x, const int8_t* scale_exp, const uint8_t* upper_cm,
                                     const uint8_t* shared_cm, void* y, float* y_f32, int64_t OUT, int64_t NB, int u,
                                     int gs, void* workspace, size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     return gemv_dispatch(x, scale_exp, upper_cm, shared_cm, y, y_f32, 1, OUT, NB, u, gs, true, workspace,
                          workspace_bytes, stream);
 }
@@ -502,6 +502,7 @@ extern "C" int msaq_wonly_gemv_batched(const void* X, const int8_t* scale_exp, c
                                        const uint8_t* shared_cm, void* Y, float* Y_f32, int64_t M, int64_t OUT,
                                        int64_t NB, int u, int gs, void* workspace, size_t workspace_bytes,
                                        void* stream) {
+    const DeviceScope device;
     return gemv_dispatch(X, scale_exp, upper_cm, shared_cm, Y, Y_f32, M, OUT, NB, u, gs, true, workspace,
                          workspace_bytes, stream);
 }
@@ -510,6 +511,7 @@ extern "C" int msaq_wonly_gemv_batched(const void* X, const int8_t* scale_exp, c
 static size_t fused_tail(int64_t M, int64_t NB) { return ((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255; }
 
 extern "C" size_t msaq_wonly_gemv_fused_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
+    const DeviceScope device;
     const size_t g = msaq_wonly_gemv_workspace(M, OUT, NB, u, gs);
     if (g == 0) return 0;
     return ((g + 255) & ~(size_t)255) + fused_tail(M, NB);
@@ -520,6 +522,7 @@ extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* ad
                                      const uint8_t* shared_cm, void* y, float* y_f32, int64_t M, int64_t OUT,
                                      int64_t NB, int u, int gs, void* workspace, size_t workspace_bytes,
                                      void* stream) {
+    const DeviceScope device;
     if (prologue < MSAQ_PRO_NONE || prologue > MSAQ_PRO_ADD_RMSNORM)
         return fail(MSAQ_ERR_ARG, "unknown prologue %d", prologue);
     if (prologue == MSAQ_PRO_NONE)
@@ -575,6 +578,7 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
                                          const uint8_t* upper_cm, const uint8_t* shared_cm, const void* residual, void* y,
                                          int64_t M, int64_t OUT, int64_t NB, int u, int gs, void* workspace,
                                          size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (prologue != MSAQ_PRO_NONE && prologue != MSAQ_PRO_RMSNORM && prologue != MSAQ_PRO_SILU_MUL)
         return fail(MSAQ_ERR_ARG, "prologue %d: none, rmsnorm or SiLU*mul", prologue);
     if (!x || !scale_exp || !upper_cm || !shared_cm || !residual || !y) return fail(MSAQ_ERR_ARG, "null pointer");
@@ -584,12 +588,13 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
     const size_t need = gemv_workspace_front(M, OUT, NB, u, gs, fused_tail(M, NB), workspace_bytes) + fused_tail(M, NB);
     if (!workspace || workspace_bytes < need)
         return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
+    int cg, cs;
     const bool ok = !((reinterpret_cast<uintptr_t>(x) & 15) | (reinterpret_cast<uintptr_t>(y) & 7) |
                       (reinterpret_cast<uintptr_t>(residual) & 7)) && M < GU_MIN_M &&
                     mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true) &&
                     // sizes whose plain GEMV is the register kernel's take its sum and add behind it
                     !(prologue == MSAQ_PRO_NONE && M > 4 && option_tensor_memory() && reg_serves(M, OUT, NB, u) &&
-                      !direct_usable(x, XP_PLAIN, M, OUT, NB, u));
+                      !direct_usable(x, XP_PLAIN, M, OUT, NB, u, &cg, &cs));
     if (ok) {
         const Prologue pro{prologue, nullptr, 0, nullptr, eps};
         return run_mma(static_cast<const __nv_bfloat16*>(x), pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB,
@@ -608,6 +613,7 @@ extern "C" int msaq_wonly_gemv_fused_push(const void* x, int prologue, const voi
                                           const uint8_t* shared_cm, int64_t M, int64_t OUT, int64_t NB, int u, int gs,
                                           void* const* peer_bufs, int rank, int world, int parity, void* workspace,
                                           size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (prologue < MSAQ_PRO_NONE || prologue > MSAQ_PRO_ADD_RMSNORM) return fail(MSAQ_ERR_ARG, "unknown prologue %d", prologue);
     if (!x || !scale_exp || !upper_cm || !shared_cm || !peer_bufs) return fail(MSAQ_ERR_ARG, "null pointer");
     if (prologue == MSAQ_PRO_ADD_RMSNORM && (!addend || !h_out))
@@ -650,8 +656,8 @@ void* g_static_ptr[64] = {};
 // handle; the address a kernel can use comes from cudaGetSymbolAddress, asked once per device
 // while that device is current.
 int static_scratch(void** out) {
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+    const int dev = current_device();
+    if (dev < 0 || dev >= 64)
         return msaq::fail(MSAQ_ERR_CUDA, "no usable current device for the static scratch");
     std::lock_guard<std::mutex> lock(g_static_mutex);
     if (!g_static_ptr[dev]) {
@@ -671,6 +677,7 @@ extern "C" size_t msaq_static_scratch_bytes(void) { return MSAQ_STATIC_SCRATCH_B
 extern "C" int msaq_wonly_gemv_wide_static(const void* x, const int8_t* scale_exp, const uint8_t* upper_cm,
                                            const uint8_t* shared_cm, void* y, float* y_f32, int64_t OUT, int64_t NB,
                                            int u, int gs, void* stream) {
+    const DeviceScope device;
     const size_t need = gemv_workspace_min(1, OUT, NB, u, gs);
     if (need == 0) return msaq::fail(MSAQ_ERR_ARG, "OUT and NB must be positive");
     if (need > MSAQ_STATIC_SCRATCH_BYTES)
@@ -685,6 +692,7 @@ extern "C" int msaq_wonly_gemv_wide_static(const void* x, const int8_t* scale_ex
 
 // ---- plain MXINT8 GEMV (the reference's matched baseline, csrc/mxint8.cu:196-253) ----------------------
 extern "C" size_t msaq_mxint8_gemv_workspace(int64_t M, int64_t OUT, int64_t NB) {
+    const DeviceScope device;
     if (M <= 0 || OUT <= 0 || NB <= 0) return 0;
     return plan_mma(M, OUT, NB, GF_MXINT8).total;
 }
@@ -692,6 +700,7 @@ extern "C" size_t msaq_mxint8_gemv_workspace(int64_t M, int64_t OUT, int64_t NB)
 extern "C" int msaq_mxint8_gemv_batched_wide(const void* X, const int8_t* scale_exp, const int8_t* qweight_cm, void* Y,
                                              float* Y_f32, int64_t M, int64_t OUT, int64_t NB, void* workspace,
                                              size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (!X || !scale_exp || !qweight_cm || !Y) return fail(MSAQ_ERR_ARG, "null pointer");
     if (M <= 0 || OUT <= 0 || NB <= 0) return fail(MSAQ_ERR_ARG, "M, OUT and NB must be positive");
     if (M > INT32_MAX || OUT > INT32_MAX || NB * BLOCK > INT32_MAX) return fail(MSAQ_ERR_ARG, "size exceeds 2^31");

@@ -8,8 +8,7 @@ template <int U, int MT>
 int launch_reg(const GemvRegArgs& a, cudaStream_t st) {
     static int configured[64] = {};                      // largest dynamic smem size set per device
     const int smem = GR_TEAMS * a.sch.stages * gr_stage_bytes(U, MT) + gr_merge_bytes(MT);
-    int dev = 0;
-    cudaGetDevice(&dev);
+    const int dev = current_device();
     if (dev >= 0 && dev < 64 && configured[dev] < smem) {
         if (cudaFuncSetAttribute(gemv_reg_kernel<U, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return fail(MSAQ_ERR_CUDA, "cannot reserve %d bytes of shared memory", smem);

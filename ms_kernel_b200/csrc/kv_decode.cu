@@ -68,8 +68,7 @@ template <int G, int FMT, int CPS>
 int launch_kv_mma_cps(const KvMmaArgs& a, int S, int Hkv, int B, cudaStream_t st) {
     static bool configured[64] = {};
     constexpr int smem = kvm_smem_bytes(FMT, CPS);
-    int dev = 0;
-    cudaGetDevice(&dev);
+    const int dev = current_device();
     if (dev >= 0 && dev < 64 && !configured[dev]) {
         if (cudaFuncSetAttribute(kv_decode_u4gs2_kernel<G, FMT, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess)
@@ -204,6 +203,7 @@ int decode_dispatch(const void* q, KvPlanes kp, KvPlanes vp, void* out, float* o
 using namespace msaq;
 
 extern "C" size_t msaq_kv_decode_workspace(int64_t B, int64_t H, int64_t Hkv, int64_t Lk, int64_t D) {
+    const DeviceScope device;
     if (B <= 0 || H <= 0 || Lk <= 0 || D <= 0) return 0;
     const KvPlan p = plan_generic(B, H, Lk);
     size_t bytes = (size_t)B * H * p.S * kv_partial_stride((int)D) * sizeof(float);
@@ -220,6 +220,7 @@ extern "C" int msaq_kv_decode_attention(const void* q, const int8_t* ks, const u
                                         float* out_f32, int64_t H, int64_t Hkv, int64_t Lk, int64_t D, int64_t NB,
                                         int u, int gs, int64_t Lcap, void* workspace, size_t workspace_bytes,
                                         void* stream) {
+    const DeviceScope device;
     return decode_dispatch(q, KvPlanes{ks, ku, kh}, KvPlanes{vs, vu, vh}, out, out_f32, nullptr, 1, H, Hkv, Lk, D, NB,
                            u, gs, Lcap, 0, QRope{}, workspace, workspace_bytes, stream);
 }
@@ -230,6 +231,7 @@ extern "C" int msaq_kv_decode_attention_batched(const void* q, const int8_t* ks,
                                                 int64_t Hkv, int64_t Lk, int64_t D, int64_t NB, int u, int gs,
                                                 int64_t Lcap, int qrot, void* workspace, size_t workspace_bytes,
                                                 void* stream) {
+    const DeviceScope device;
     return decode_dispatch(q, KvPlanes{ks, ku, kh}, KvPlanes{vs, vu, vh}, out, out_f32, seq_lens, B, H, Hkv, Lk, D, NB,
                            u, gs, Lcap, qrot, QRope{}, workspace, workspace_bytes, stream);
 }
@@ -241,6 +243,7 @@ extern "C" int msaq_kv_decode_attention_rope(const void* q, const int8_t* ks, co
                                              const float* rope_cos, const float* rope_sin, int64_t rope_rows,
                                              int64_t q_pos, const int32_t* q_pos_per_seq, void* workspace,
                                              size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     return decode_dispatch(q, KvPlanes{ks, ku, kh}, KvPlanes{vs, vu, vh}, out, out_f32, seq_lens, B, H, Hkv, Lk, D, NB,
                            u, gs, Lcap, qrot, QRope{Rope{rope_cos, rope_sin, rope_rows}, q_pos, q_pos_per_seq}, workspace,
                            workspace_bytes, stream);
@@ -253,6 +256,7 @@ extern "C" int msaq_kv_decode_attention_append(const void* q, const void* k_new,
                                                const float* rope_cos, const float* rope_sin, int64_t rope_rows,
                                                int64_t pos, const int32_t* pos_per_seq, void* workspace,
                                                size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (!k_new || !v_new) return fail(MSAQ_ERR_ARG, "null pointer");
     if ((reinterpret_cast<uintptr_t>(k_new) | reinterpret_cast<uintptr_t>(v_new)) & 7)
         return fail(MSAQ_ERR_ARG, "k_new and v_new must be 8-byte aligned");
@@ -272,6 +276,7 @@ extern "C" int msaq_mxint8_kv_decode_batched(const void* q, const int8_t* ks, co
                                              const int8_t* vq, void* out, float* out_f32, const int32_t* seq_lens,
                                              int64_t B, int64_t H, int64_t Hkv, int64_t Lk, int64_t D, int64_t NB,
                                              int64_t Lcap, void* workspace, size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (!q || !ks || !kq || !vs || !vq || !out) return fail(MSAQ_ERR_ARG, "null pointer");
     if (B <= 0 || H <= 0 || Hkv <= 0 || Lk <= 0) return fail(MSAQ_ERR_ARG, "B, H, Hkv and Lk must be positive");
     if (H % Hkv) return fail(MSAQ_ERR_ARG, "H (%lld) must be a multiple of Hkv (%lld)", (long long)H, (long long)Hkv);

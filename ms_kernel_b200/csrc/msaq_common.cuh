@@ -49,6 +49,16 @@ size_t gemv_workspace_front(int64_t M, int64_t OUT, int64_t NB, int u, int gs, s
 int fail(int code, const char* fmt, ...);
 int check_launch(const char* what);
 void count_launch(int n = 1);
+// The current device.  Asking the runtime costs a few tenths of a microsecond and a call's plans want it dozens of times (a
+// workspace query came to several microseconds of host time), so an entry point opens a DeviceScope, within which the answer is
+// kept; nothing is kept from one call to the next.
+struct DeviceScope {
+    DeviceScope();
+    ~DeviceScope();
+    DeviceScope(const DeviceScope&) = delete;
+    DeviceScope& operator=(const DeviceScope&) = delete;
+};
+int current_device();         // -1 if the runtime cannot say
 int sm_count();               // SM count of the current device (cached per device)
 int require_sm100();          // MSAQ_OK or MSAQ_ERR_DEVICE
 bool option_chained_launch(); // kernels are launched with programmatic stream serialisation

@@ -176,6 +176,7 @@ extern "C" int msaq_quant_act(const void* X, int8_t* qX, int8_t* sa_exp, int64_t
 }
 
 extern "C" size_t msaq_wa_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
+    const DeviceScope device;
     const size_t g = msaq_wonly_gemv_workspace(M, OUT, NB, u, gs);
     if (g == 0) return 0;
     return ((g + 255) & ~(size_t)255) + (((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255);
@@ -184,6 +185,7 @@ extern "C" size_t msaq_wa_gemv_workspace(int64_t M, int64_t OUT, int64_t NB, int
 extern "C" int msaq_wa_gemv_batched(const void* X, const int8_t* scale_exp, const uint8_t* upper_cm,
                                     const uint8_t* shared_cm, void* Y, float* Y_f32, int64_t M, int64_t OUT, int64_t NB,
                                     int u, int gs, void* workspace, size_t workspace_bytes, void* stream) {
+    const DeviceScope device;
     if (M <= 0 || OUT <= 0 || NB <= 0) return fail(MSAQ_ERR_ARG, "M, OUT and NB must be positive");
     const size_t tail = ((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255;
     const size_t g = gemv_workspace_front(M, OUT, NB, u, gs, tail, workspace_bytes), need = g + tail;
