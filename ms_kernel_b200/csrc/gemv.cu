@@ -628,7 +628,7 @@ extern "C" int msaq_wonly_gemv_fused_push(const void* x, int prologue, const voi
         !mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true))
         return fail(MSAQ_ERR_UNSUPPORTED, "the push is built into the integer-MMA GEMV only (u=4, gs=2, up to 8 rows, aligned "
                                           "column-major planes): run the GEMV and msaq_peer_exchange separately");
-    const size_t need = msaq_wonly_gemv_fused_workspace(M, OUT, NB, u, gs);
+    const size_t need = ((gemv_workspace_min(M, OUT, NB, u, gs) + 255) & ~(size_t)255) + fused_tail(M, NB);      // as the GEMV without the push
     if (workspace_bytes < need) return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     PeerPush push{};
     for (int r = 0; r < world; ++r) {

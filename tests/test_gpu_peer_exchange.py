@@ -127,6 +127,35 @@ def test_argument_checks():
     assert _lib.lib().msaq_peer_exchange_bytes(9, n) == 0
 
 
+def test_push_takes_the_smallest_workspace_of_the_gemv_without_it():
+    """512 x 8192 at eight rows: the plain product can also use the register kernel's larger scratch, the push never does."""
+    import ctypes
+    import re
+    from ms_kernel_b200 import ops, pack
+    L = _lib.lib()
+    M, OUT, K = 8, 512, 8192
+    lin = ops.PackedLinear(pack.pack_weight((torch.randn((OUT, K), device="cuda") * 0.02).to(torch.bfloat16), 4, 2), "cuda")
+    x = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    y = torch.empty((M, OUT), dtype=torch.bfloat16, device="cuda")
+    planes = (lin.scale_exp.data_ptr(), lin.upper_cm.data_ptr(), lin.shared_cm.data_ptr())
+    rc = L.msaq_wonly_gemv_fused(x.data_ptr(), 1, None, 0, 1e-5, None, *planes, y.data_ptr(), None, M, OUT, K // 32, 4, 2, None, 0, None)
+    assert rc == -3
+    need = int(re.search(rb"of (\d+) bytes", L.msaq_last_error()).group(1))
+    assert need < L.msaq_wonly_gemv_fused_workspace(M, OUT, K // 32, 4, 2)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    bufs = _bufs(2, M * OUT, torch.device("cuda", 0))
+    ptrs = (ctypes.c_void_p * 2)(*[b.data_ptr() for b in bufs])
+
+    def push(nbytes):
+        return L.msaq_wonly_gemv_fused_push(x.data_ptr(), 0, None, 0, 1e-5, None, *planes, M, OUT, K // 32, 4, 2, ptrs, 0, 2, 0,
+                                            ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+    assert push(need) == 0, L.msaq_last_error()
+    assert push(need - 256) == -3
+    torch.cuda.synchronize()
+    got = _slot(bufs[1], 2, M * OUT, 0, 0)[:, 0::2].contiguous().view(torch.float32).view(M, OUT)
+    assert torch.equal(got.to(torch.bfloat16), lin.fwd(x))
+
+
 @pytest.mark.parametrize("OUT,K,M,prologue", [(8192, 1024, 1, 0), (8192, 3584, 1, 2), (4096, 2048, 4, 0), (8192, 4096, 8, 2),
                                               (1024, 256, 1, 0)])
 def test_gemv_with_the_push_inside(OUT, K, M, prologue):
