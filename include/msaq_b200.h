@@ -372,8 +372,8 @@ int msaq_peer_exchange(const float* partial, const void* residual, void* out, vo
  * y = bf16(residual + bf16(W . pro(x))): msaq_wonly_gemv_fused (prologue none, rmsnorm or SiLU*mul) with the
  * residual add of a decoder layer's last projection done by the GEMV's finishing warps -- the same two roundings
  * as the GEMV followed by msaq_add_residual, one launch fewer.  residual and y bf16 [M, OUT]; y may be the
- * residual's own memory (every output is read before it is written, by the same thread).  Formats and sizes the
- * integer-MMA kernel does not serve run the two steps as separate kernels.
+ * residual's own memory.  u = 4, gs = 2 up to eight rows (aligned column-major planes); every other format and size runs the
+ * two steps as separate kernels, which in the residual's own memory takes all of msaq_wonly_gemv_fused_workspace.
  */
 int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps, const int8_t* scale_exp,
                               const uint8_t* upper_cm, const uint8_t* shared_cm, const void* residual, void* y,

@@ -255,8 +255,21 @@ RegPlan plan_reg(int64_t M, int64_t OUT, int64_t NB, int u) {
     return p;
 }
 
+// Whether the register kernel can serve these arguments (and is the one for their sizes): X is read and the outputs are
+// stored sixteen bytes at a time, and the workspace has to hold its partial sums.
+bool reg_usable(const void* X, const int8_t* se, const uint8_t* up, const uint8_t* sh, const void* Y, const float* Yf, int64_t M,
+                int64_t OUT, int64_t NB, int u, int gs, bool cm, const void* ws, size_t ws_bytes, RegPlan* p) {
+    if (!option_tensor_memory() || !umma_eligible(OUT, u, gs, cm) || !reg_serves(M, OUT, NB, u)) return false;
+    if ((reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(sh) | reinterpret_cast<uintptr_t>(se) | reinterpret_cast<uintptr_t>(ws) |
+         reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15)
+        return false;
+    *p = plan_reg(M, OUT, NB, u);
+    return ws_bytes >= p->total;
+}
+
+// `res` (up to eight rows): the residual add behind the product, see GemvRegArgs.
 int run_reg(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y, float* Yf,
-            int64_t M, int64_t OUT, int64_t NB, int u, const RegPlan& p, void* ws, cudaStream_t st) {
+            int64_t M, int64_t OUT, int64_t NB, int u, const RegPlan& p, void* ws, cudaStream_t st, const void* res = nullptr) {
     uint8_t* base = static_cast<uint8_t*>(ws);
     int* status = reinterpret_cast<int*>(base);
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(base + 256);
@@ -267,8 +280,8 @@ int run_reg(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const u
     // many of them in hand one after another, and a second, fully parallel launch is faster (4096x4096, 16 rows: 18.2 us
     // inside, 14.4 us with the launch; 1024x8192, eight rows: 14.0 us inside, 17.2 us with it).
     const int combine = M > 8;
-    GemvRegArgs a{se, up, sh, X, partial, counters, status, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf, 0, (int)M,
-                  (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(), tag, combine};
+    GemvRegArgs a{se, up, sh, X, partial, counters, status, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf,
+                  static_cast<const __nv_bfloat16*>(res), 0, (int)M, (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(), tag, combine};
     const int rc = gemv_reg_launch(a, u, p.mt, st);
     if (rc || !combine || (sch.units() % sch.grid == 0 && (sch.units() / sch.grid) % sch.nb == 0)) return rc;
     const int64_t quads = M * (OUT / 4);
@@ -433,11 +446,9 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     int cg = 1, cs = 1;
     if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u, &cg, &cs))
         return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, cg, cs, nullptr, nullptr, st);
-    // up to 64 rows on register operands, where X can be read sixteen bytes at a time and the workspace holds its partials
-    if (tm_ok && reg_serves(M, OUT, NB, u) && !(reinterpret_cast<uintptr_t>(X) & 15)) {
-        const RegPlan p = plan_reg(M, OUT, NB, u);
-        if (ws_bytes >= p.total) return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, p, ws, st);
-    }
+    RegPlan reg;
+    if (reg_usable(X, se, up, sh, Y, Yf, M, OUT, NB, u, gs, cm, ws, ws_bytes, &reg))
+        return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, reg, ws, st);
     // u = 4 keeps up to eight rows on the integer-MMA kernel
     if (tm_ok && (u != 4 || M >= GU_MIN_M)) return run_umma(x, se, up, sh, Y, Yf, M, OUT, NB, u, ws, st);
     // the integer-MMA kernel's finishing warps store four outputs at a time: 8-byte aligned bf16, 16-byte aligned fp32
@@ -508,13 +519,15 @@ extern "C" int msaq_wonly_gemv_batched(const void* X, const int8_t* scale_exp, c
 }
 
 // ---- GEMV with the layer glue in front of it fused into the activation staging ---------------
+// bytes of bf16 [rows][cols], rounded up: the glue's output (and, for a residual add in place, the product) behind the GEMV's scratch
 static size_t fused_tail(int64_t M, int64_t NB) { return ((size_t)M * NB * BLOCK * 2 + 255) & ~(size_t)255; }
+static size_t product_tail(int64_t M, int64_t OUT) { return ((size_t)M * OUT * 2 + 255) & ~(size_t)255; }
 
 extern "C" size_t msaq_wonly_gemv_fused_workspace(int64_t M, int64_t OUT, int64_t NB, int u, int gs) {
     const DeviceScope device;
     const size_t g = msaq_wonly_gemv_workspace(M, OUT, NB, u, gs);
     if (g == 0) return 0;
-    return ((g + 255) & ~(size_t)255) + fused_tail(M, NB);
+    return ((g + 255) & ~(size_t)255) + fused_tail(M, NB) + product_tail(M, OUT);
 }
 
 extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* addend, int addend_is_f32, float eps,
@@ -585,26 +598,40 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
     if (M <= 0 || OUT <= 0 || NB <= 0) return fail(MSAQ_ERR_ARG, "M, OUT and NB must be positive");
     if (M > INT32_MAX || OUT > INT32_MAX || NB * BLOCK > INT32_MAX / 2) return fail(MSAQ_ERR_ARG, "size exceeds 2^31");
     if (int rc = require_sm100()) return rc;
-    const size_t need = gemv_workspace_front(M, OUT, NB, u, gs, fused_tail(M, NB), workspace_bytes) + fused_tail(M, NB);
-    if (!workspace || workspace_bytes < need)
-        return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
-    int cg, cs;
+    size_t tail = fused_tail(M, NB), front = gemv_workspace_front(M, OUT, NB, u, gs, tail, workspace_bytes);
+    if (!workspace || workspace_bytes < front + tail)
+        return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", front + tail, workspace ? workspace_bytes : (size_t)0);
+    const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool ok = !((reinterpret_cast<uintptr_t>(x) & 15) | (reinterpret_cast<uintptr_t>(y) & 7) |
                       (reinterpret_cast<uintptr_t>(residual) & 7)) && M < GU_MIN_M &&
-                    mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true) &&
-                    // sizes whose plain GEMV is the register kernel's take its sum and add behind it
-                    !(prologue == MSAQ_PRO_NONE && M > 4 && option_tensor_memory() && reg_serves(M, OUT, NB, u) &&
-                      !direct_usable(x, XP_PLAIN, M, OUT, NB, u, &cg, &cs));
+                    mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true);
     if (ok) {
+        // without a prologue the sum is the plain GEMV's, whichever kernel that is
+        int cg, cs;
+        RegPlan reg;
+        if (prologue == MSAQ_PRO_NONE && M > 4 && !direct_usable(x, XP_PLAIN, M, OUT, NB, u, &cg, &cs) &&
+            reg_usable(x, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, u, gs, true, workspace, workspace_bytes, &reg))
+            return run_reg(xb, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, u, reg, workspace, st, residual);
         const Prologue pro{prologue, nullptr, 0, nullptr, eps};
-        return run_mma(static_cast<const __nv_bfloat16*>(x), pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB,
-                       workspace, static_cast<cudaStream_t>(stream), GF_MSAQ_U4, nullptr, residual);
+        return run_mma(xb, pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, workspace, st, GF_MSAQ_U4, nullptr, residual);
     }
-    // every other format and size: the same two steps as separate kernels (identical roundings)
-    if (int rc = msaq_wonly_gemv_fused(x, prologue, nullptr, 0, eps, nullptr, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT,
+    // Every other format and size: the same two steps as separate kernels (identical roundings).  With the residual in y's own
+    // memory the product goes to the end of the workspace first.
+    const uintptr_t y0 = reinterpret_cast<uintptr_t>(y), r0 = reinterpret_cast<uintptr_t>(residual), n = (uintptr_t)M * OUT * 2;
+    void* product = y;
+    if (y0 < r0 + n && r0 < y0 + n) {
+        front = gemv_workspace_front(M, OUT, NB, u, gs, tail + product_tail(M, OUT), workspace_bytes);
+        if (workspace_bytes < front + tail + product_tail(M, OUT))
+            return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed for a residual add in place, %zu given",
+                        front + tail + product_tail(M, OUT), workspace_bytes);
+        product = static_cast<uint8_t*>(workspace) + front + tail;
+        workspace_bytes = front + tail;
+    }
+    if (int rc = msaq_wonly_gemv_fused(x, prologue, nullptr, 0, eps, nullptr, scale_exp, upper_cm, shared_cm, product, nullptr, M, OUT,
                                        NB, u, gs, workspace, workspace_bytes, stream))
         return rc;
-    return msaq_add_residual(residual, y, 0, y, M * OUT, stream);
+    return msaq_add_residual(residual, product, 0, y, M * OUT, stream);
 }
 
 // ---- GEMV of a row-parallel projection with the exchange's push inside --------------------

@@ -252,6 +252,7 @@ struct GemvRegArgs {
     int* sticky;
     __nv_bfloat16* y;
     float* y_f32;                // optional
+    const __nv_bfloat16* res;    // optional (up to eight rows): y = bf16(res + bf16(W x)); may be y itself
     int m0, rows, OUT, NB;
     GemvSchedule sch;            // sch.nb counts units of GR_KB K blocks
     uint32_t max_polls;
@@ -440,7 +441,9 @@ gemv_reg_kernel(const GemvRegArgs a) {
                                 const int o = o0 + q * GM_GROUP + r0 + (i >> 1) * 8;
                                 if (nslots == 1) {
                                     const int64_t yo = (int64_t)(a.m0 + m) * a.OUT + o;
-                                    a.y[yo] = __float2bfloat16_rn(v);
+                                    __nv_bfloat16 y = __float2bfloat16_rn(v);
+                                    if (MT == 1 && a.res) y = __float2bfloat16_rn(__bfloat162float(a.res[yo]) + __bfloat162float(y));
+                                    a.y[yo] = y;
                                     if (a.y_f32) a.y_f32[yo] = v;
                                 } else {
                                     a.partial[((int64_t)slot * a.rows + m) * a.OUT + o] = v;
@@ -495,6 +498,13 @@ gemv_reg_kernel(const GemvRegArgs a) {
                             if (poison) sum.x = sum.y = sum.z = sum.w = nan;
                             const int64_t y0 = (int64_t)a.m0 * a.OUT + e;
                             if (a.y_f32) *reinterpret_cast<float4*>(a.y_f32 + y0) = sum;
+                            if (MT == 1 && a.res) {        // the projection rounds to bf16 first, as the unfused add sees it
+                                const uint2 rb = *reinterpret_cast<const uint2*>(a.res + y0);
+                                sum.x = bf16_lo(rb.x) + __bfloat162float(__float2bfloat16_rn(sum.x));
+                                sum.y = bf16_hi(rb.x) + __bfloat162float(__float2bfloat16_rn(sum.y));
+                                sum.z = bf16_lo(rb.y) + __bfloat162float(__float2bfloat16_rn(sum.z));
+                                sum.w = bf16_hi(rb.y) + __bfloat162float(__float2bfloat16_rn(sum.w));
+                            }
                             const __nv_bfloat162 lo = __floats2bfloat162_rn(sum.x, sum.y), hi = __floats2bfloat162_rn(sum.z, sum.w);
                             *reinterpret_cast<uint2*>(a.y + y0) =
                                 make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));

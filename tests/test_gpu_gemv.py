@@ -261,3 +261,36 @@ def test_residual_add_behind_the_gemv_is_bit_equal_to_the_two_steps(rng, OUT, K,
     got = lin.fwd_fused_add(x, prologue, h)
     torch.cuda.synchronize()
     assert torch.equal(got, want.reshape(M, OUT))
+
+
+@pytest.mark.parametrize("u,gs,M,OUT,K,prologue", [(4, 2, 1, 512, 256, 0), (4, 2, 6, 512, 256, 0), (4, 2, 5, 9616, 96, 0),
+                                                   (4, 2, 8, 9616, 1056, 0), (4, 2, 8, 512, 256, 2), (4, 2, 12, 512, 256, 0),
+                                                   (4, 2, 20, 528, 256, 1), (4, 2, 70, 528, 256, 0), (3, 2, 2, 528, 256, 0),
+                                                   (2, 2, 1, 528, 256, 2), (4, 4, 3, 40, 96, 1)])
+def test_residual_add_in_the_residuals_own_memory(u, gs, M, OUT, K, prologue):
+    """y may be the residual: the result is that of the call with an output of its own, on every kernel -- inside it (direct,
+    register-operand with whole and with split tiles, integer) and as two kernels, which need the whole workspace."""
+    from ms_kernel_b200 import _lib, ops, pack
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(OUT + K + M + u)
+    W = (torch.randn((OUT, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    lin = ops.PackedLinear(pack.pack_weight(W, u, gs), "cuda")
+    x = torch.randn((M, (2 if prologue == 2 else 1) * K), generator=g, device="cuda").to(torch.bfloat16)
+    res = torch.randn((M, OUT), generator=g, device="cuda").to(torch.bfloat16)
+    y = lin.fwd_fused(x, prologue) if prologue else lin.fwd(x)
+    want = torch.ops.msaq.add_residual(res, y.reshape(M, OUT).contiguous())
+    assert torch.equal(lin.fwd_fused_add(x, prologue, res), want)
+    wsb = L.msaq_wonly_gemv_fused_workspace(M, OUT, K // 32, u, gs)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+
+    def in_place(nbytes):
+        got = res.clone()
+        rc = L.msaq_wonly_gemv_fused_add(x.data_ptr(), prologue, 1e-5, lin.scale_exp.data_ptr(), lin.upper_cm.data_ptr(),
+                                         lin.shared_cm.data_ptr(), got.data_ptr(), got.data_ptr(), M, OUT, K // 32, u, gs,
+                                         ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return rc, got
+    rc, got = in_place(wsb)
+    assert rc == 0 and torch.equal(got, want)
+    rc, got = in_place(1024)                       # too little: refused, nothing touched
+    assert rc == -3 and torch.equal(got, res)
