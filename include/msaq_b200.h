@@ -148,7 +148,8 @@ int msaq_wonly_gemv_batched(const void* X, const int8_t* scale_exp, const uint8_
  * separate entry points msaq_rmsnorm / msaq_silu_mul / msaq_add_residual round it.  Column-major planes, any
  * (u, gs); formats outside the tuned path run the glue as separate kernels into the workspace tail.
  * h_out must not overlap x or addend (MSAQ_ERR_ARG): there is no in-place residual update.
- * A non-finite activation (Inf or NaN) turns its whole output row into NaN.
+ * A non-finite activation (Inf or NaN) turns its whole output row into NaN at u = 4, gs = 2 up to eight rows (this entry point
+ * and the GEMVs above); elsewhere it goes through the products as in floating-point arithmetic.
  */
 #define MSAQ_PRO_NONE 0
 #define MSAQ_PRO_RMSNORM 1

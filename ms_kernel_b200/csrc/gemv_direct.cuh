@@ -423,13 +423,7 @@ gemv_direct_bf16_kernel(const GemvDirectArgs a) {
             uint32_t b[MT][4];
 #pragma unroll
             for (int n = 0; n < MT; ++n) {
-                uint4 x = xc[d][n];
-                if (U == 4 && MT == 1) {    // Inf becomes NaN, and with it the whole row, as in the integer kernels
-                    x.x = hfma2_bf16(x.x, 0u, x.x);
-                    x.y = hfma2_bf16(x.y, 0u, x.y);
-                    x.z = hfma2_bf16(x.z, 0u, x.z);
-                    x.w = hfma2_bf16(x.w, 0u, x.w);
-                }
+                const uint4 x = gr_finite_or_nan<U, MT>(xc[d][n]);
                 b[n][0] = prmt(x.x, x.z, 0x5410u);
                 b[n][1] = prmt(x.x, x.z, 0x7632u);
                 b[n][2] = prmt(x.y, x.w, 0x5410u);

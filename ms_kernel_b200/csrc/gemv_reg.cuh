@@ -165,21 +165,35 @@ __device__ __forceinline__ void gr_decode_row(uint32_t ub, uint32_t sb, uint32_t
     gr_decode<U>(r, ln, k, w);
 }
 
+// u = 4 up to eight rows: an Inf becomes NaN, and with it the whole output row, as in the integer kernels that share these
+// row counts (their fixed point cannot hold it), so that the result does not depend on the kernel a size falls to.  Four more
+// instructions per 32-block and eight rows.
+template <int U, int MT>
+__device__ __forceinline__ uint4 gr_finite_or_nan(uint4 x) {
+    if constexpr (U == 4 && MT == 1) {
+        x.x = hfma2_bf16(x.x, 0u, x.x);
+        x.y = hfma2_bf16(x.y, 0u, x.y);
+        x.z = hfma2_bf16(x.z, 0u, x.z);
+        x.w = hfma2_bf16(x.w, 0u, x.w);
+    }
+    return x;
+}
+
 // K block J of a stage: its activation fragments and the weights of the warp's groups, in the order that leaves fewer registers
 // in use.  Every group is computed: columns beyond the matrix (a ragged last tile) come out as garbage that is not stored.
-template <int MT, int J, int N>
+template <int U, int MT, int J, int N>
 __device__ __forceinline__ void gr_activation(uint32_t xb, uint32_t (&b)[4]) {
-    const uint4 x = lds128<N * 8 * GR_XROW + J * 64>(xb);
+    const uint4 x = gr_finite_or_nan<U, MT>(lds128<N * 8 * GR_XROW + J * 64>(xb));
     b[0] = prmt(x.x, x.z, 0x5410u);
     b[1] = prmt(x.x, x.z, 0x7632u);
     b[2] = prmt(x.y, x.w, 0x5410u);
     b[3] = prmt(x.y, x.w, 0x7632u);
 }
-template <int MT, int J, int N>
+template <int U, int MT, int J, int N>
 __device__ __forceinline__ void gr_activations(uint32_t xb, uint32_t (&b)[MT][4]) {
     if constexpr (N < MT) {
-        gr_activation<MT, J, N>(xb, b[N]);
-        gr_activations<MT, J, N + 1>(xb, b);
+        gr_activation<U, MT, J, N>(xb, b[N]);
+        gr_activations<U, MT, J, N + 1>(xb, b);
     }
 }
 template <int U, int MT, int J, int Q>
@@ -210,16 +224,16 @@ __device__ __forceinline__ void gr_groups(uint32_t ub, uint32_t sb, uint32_t eb,
         gr_groups<U, MT, J, Q + 1>(ub, sb, eb, ln, k, b, acc);
     }
 }
-template <int MT, int J, int N>
+template <int U, int MT, int J, int N>
 __device__ __forceinline__ void gr_rows(uint32_t xb, const uint32_t (&w0)[4], const uint32_t (&w1)[4], float (&acc)[MT][4]) {
     if constexpr (N < MT) {                                                   // four n-tiles at a time
         uint32_t b[4][4];
-        gr_activation<MT, J, N>(xb, b[0]);
-        gr_activation<MT, J, N + 1>(xb, b[1]);
-        gr_activation<MT, J, N + 2>(xb, b[2]);
-        gr_activation<MT, J, N + 3>(xb, b[3]);
+        gr_activation<U, MT, J, N>(xb, b[0]);
+        gr_activation<U, MT, J, N + 1>(xb, b[1]);
+        gr_activation<U, MT, J, N + 2>(xb, b[2]);
+        gr_activation<U, MT, J, N + 3>(xb, b[3]);
         gr_mma<4, 4>(&acc[N], w0, w1, b);
-        gr_rows<MT, J, N + 4>(xb, w0, w1, acc);
+        gr_rows<U, MT, J, N + 4>(xb, w0, w1, acc);
     }
 }
 template <int U, int MT, int J>
@@ -229,12 +243,12 @@ __device__ __forceinline__ void gr_blocks(int nblk, uint32_t ub, uint32_t sb, ui
         if (J < nblk) {
             if constexpr (gr_groups_of(MT) > 1) {
                 uint32_t b[MT][4];
-                gr_activations<MT, J, 0>(xb, b);
+                gr_activations<U, MT, J, 0>(xb, b);
                 gr_groups<U, MT, J, 0>(ub, sb, eb, ln, k, b, acc);
             } else {
                 uint32_t w0[4], w1[4];
                 gr_weights<U, MT, J, 0>(ub, sb, eb, ln, k, w0, w1);
-                gr_rows<MT, J, 0>(xb, w0, w1, acc[0]);
+                gr_rows<U, MT, J, 0>(xb, w0, w1, acc[0]);
             }
         }
         gr_blocks<U, MT, J + 1>(nblk, ub, sb, eb, xb, ln, k, acc);

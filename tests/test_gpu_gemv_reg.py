@@ -90,3 +90,15 @@ def test_wait_gives_up_and_next_call_is_correct(rng, u, M):
     got2, gotf2 = cabi.gemv("batched", x, pd, M=M)
     cabi.check_output(got2, gotf2, ref, MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
     assert _status() == 0
+
+
+@pytest.mark.parametrize("bad", (float("inf"), float("-inf"), float("nan")))
+@pytest.mark.parametrize("M,OUT,K", [(5, 9616, 96), (8, 9616, 1056), (6, 9616, 544)])
+def test_non_finite_activation_gives_a_nan_row(rng, bad, M, OUT, K):
+    """u = 4, five to eight rows, more columns than one wave of the direct kernels: the row is NaN as a whole, as everywhere
+    up to eight rows of u = 4; the other rows are untouched."""
+    import cabi
+    X, p = _case(rng, OUT, K, 4, M)
+    X[M - 2, K - 3] = bad
+    _, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    assert np.isnan(gotf[M - 2]).all() and np.isfinite(np.delete(gotf, M - 2, 0)).all()
