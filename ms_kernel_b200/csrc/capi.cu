@@ -1,6 +1,5 @@
 // Error plumbing, launch accounting and device queries shared by the entry points.
 #include <atomic>
-#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -56,7 +55,6 @@ std::atomic<int> g_opt_tmem{1};
 std::atomic<int> g_opt_polls{1 << 20};
 std::atomic<int> g_opt_inkernel{1};
 std::atomic<int> g_opt_early{0};
-std::atomic<uint32_t> g_call_tag{0};
 std::atomic<int> g_opt_skip{-1};
 
 // One status word per GPU that loads the library: kernels OR a bit into it when a bounded wait
@@ -67,21 +65,6 @@ std::atomic<int*> g_sticky_ptr[64];
 
 bool option_early_weights() { return g_opt_early.load(std::memory_order_relaxed) != 0; }
 bool option_inkernel_staging() { return g_opt_inkernel.load(std::memory_order_relaxed) != 0; }
-
-uint32_t next_call_tag() {
-    uint32_t t = g_call_tag.load(std::memory_order_relaxed);
-    if (t == 0) {
-        // first use: start somewhere unpredictable, so that whatever a fresh workspace holds is unlikely to look like a tag
-        uint32_t seed = (uint32_t)std::chrono::steady_clock::now().time_since_epoch().count() * 2654435761u;
-        seed ^= (uint32_t)(uintptr_t)&g_call_tag;
-        uint32_t expected = 0;
-        g_call_tag.compare_exchange_strong(expected, seed | 1u);
-    }
-    for (;;) {
-        t = (g_call_tag.fetch_add(1, std::memory_order_relaxed) + 1) & 0x7FFFFFFFu;      // 31 bits: the top bit marks "being cleared"
-        if (t != 0) return t;
-    }
-}
 
 unsigned option_wait_polls() { return (unsigned)g_opt_polls.load(std::memory_order_relaxed); }
 int option_test_skip_stage() { return g_opt_skip.load(std::memory_order_relaxed); }

@@ -22,7 +22,7 @@ namespace {
 struct MmaPlan {
     GemvSchedule sch;        // sch.nb counts units of `kb` K blocks
     int kb;
-    size_t xprep_off, xprep_bytes, partial_off, total;      // status word at 0, counters at 256, then these
+    size_t xprep_off, xprep_bytes, partial_off, total;      // counters at 256, then these
 };
 
 bool mma_eligible(int64_t OUT, int u, int gs, bool cm) { return cm && u == 4 && gs == 2 && OUT % 16 == 0; }
@@ -74,7 +74,7 @@ MmaPlan plan_mma(int64_t M, int64_t OUT, int64_t NB, int fmt = GF_MSAQ_U4) {
     s.stages = stages;
     p.xprep_bytes = ((size_t)NB * passes * GM_XREC + 255) & ~(size_t)255;
     const size_t ctl = (256 + (size_t)s.col_tiles * GM_WARPS * sizeof(unsigned long long) + 255) & ~(size_t)255;
-    p.xprep_off = ctl > WS_CTL_BYTES ? ctl : WS_CTL_BYTES;            // the control region: status word, then the tile counters
+    p.xprep_off = ctl > WS_CTL_BYTES ? ctl : WS_CTL_BYTES;            // the control region: the tile counters
     p.partial_off = p.xprep_off + p.xprep_bytes;
     p.total = p.partial_off + (((size_t)s.max_slots * rows * OUT * sizeof(float) + 255) & ~(size_t)255);
     return p;
@@ -205,7 +205,7 @@ int run_umma(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const 
             const int64_t quads = (int64_t)rows * (OUT / 4);
             launch_chained(gemv_umma_combine_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st,
                            static_cast<const float*>(partial), static_cast<const int*>(status),
-                           static_cast<__nv_bfloat16*>(Y), Yf, sch, (int)m0, rows, (int)OUT, 0);
+                           static_cast<__nv_bfloat16*>(Y), Yf, sch, (int)m0, rows, (int)OUT);
             count_launch();
             if (int rc = check_launch("gemv_umma_combine")) return rc;
         }
@@ -271,23 +271,21 @@ bool reg_usable(const void* X, const int8_t* se, const uint8_t* up, const uint8_
 int run_reg(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y, float* Yf,
             int64_t M, int64_t OUT, int64_t NB, int u, const RegPlan& p, void* ws, cudaStream_t st, const void* res = nullptr) {
     uint8_t* base = static_cast<uint8_t*>(ws);
-    int* status = reinterpret_cast<int*>(base);
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(base + 256);
     float* partial = reinterpret_cast<float*>(base + p.partial_off);
     const GemvSchedule& sch = p.sch;
-    const uint32_t tag = next_call_tag();
     // Split tiles: up to eight rows the warp that arrives last at a tile adds the partial sums up; above, it would have too
     // many of them in hand one after another, and a second, fully parallel launch is faster (4096x4096, 16 rows: 18.2 us
     // inside, 14.4 us with the launch; 1024x8192, eight rows: 14.0 us inside, 17.2 us with it).
     const int combine = M > 8;
-    GemvRegArgs a{se, up, sh, X, partial, counters, status, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf,
-                  static_cast<const __nv_bfloat16*>(res), 0, (int)M, (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(), tag, combine};
+    GemvRegArgs a{se, up, sh, X, partial, counters, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf,
+                  static_cast<const __nv_bfloat16*>(res), 0, (int)M, (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(), combine};
     const int rc = gemv_reg_launch(a, u, p.mt, st);
     if (rc || !combine || (sch.units() % sch.grid == 0 && (sch.units() / sch.grid) % sch.nb == 0)) return rc;
     const int64_t quads = M * (OUT / 4);
     launch_chained(gemv_umma_combine_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, st,
-                   static_cast<const float*>(partial), static_cast<const int*>(status), static_cast<__nv_bfloat16*>(Y), Yf,
-                   sch, 0, (int)M, (int)OUT, (int)tag);
+                   static_cast<const float*>(partial), static_cast<const int*>(nullptr), static_cast<__nv_bfloat16*>(Y), Yf,
+                   sch, 0, (int)M, (int)OUT);
     count_launch();
     return check_launch("gemv_umma_combine");
 }
@@ -346,7 +344,6 @@ int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const
         return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, cg, cs, push, res, st);
     const MmaPlan p = plan_mma(M, OUT, NB, fmt);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    int* status = reinterpret_cast<int*>(base);
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(base + 256);
     uint8_t* xprep = base + p.xprep_off;
     float* partial = reinterpret_cast<float*>(base + p.partial_off);
@@ -379,7 +376,6 @@ int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const
         const long long table = max_iter * p.kb * GM_XREC;
         const bool in_kernel = fmt == GF_MSAQ_U4 && passes == 1 && pro.mode == XP_PLAIN && option_inkernel_staging() &&
                                table <= GM_MAX_TABLE;
-        const uint32_t tag = next_call_tag();
         if (in_kernel) {
             const int per_sm = (sch.grid + sm_count() - 1) / sm_count();
             int stages = (200 * 1024 / per_sm - (int)table) / (p.kb * gm_stage_bytes(sch.tc, passes, fmt));
@@ -387,9 +383,9 @@ int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const
         } else if (int rc = launch_xprep(xa, pro.mode, (unsigned)((warps * 32 + 127) / 128), st)) {
             return rc;
         }
-        GemvMmaArgs a{se, up, sh, xprep, partial, counters, status, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf,
+        GemvMmaArgs a{se, up, sh, xprep, partial, counters, sticky_status(), static_cast<__nv_bfloat16*>(Y), Yf,
                       (int)m0, rows, (int)OUT, (int)NB, sch, option_wait_polls(), option_test_skip_stage(),
-                      in_kernel ? pro.mode : -1, xa.X, xa.R, xa.h_out, (int)ldx, pro.r_is_f32, pro.eps, tag,
+                      in_kernel ? pro.mode : -1, xa.X, xa.R, xa.h_out, (int)ldx, pro.r_is_f32, pro.eps,
                       in_kernel ? (int)table : 0, 0, option_early_weights() ? 1 : 0, push ? *push : PeerPush{},
                       static_cast<const __nv_bfloat16*>(res)};
         // the ring depth was planned for the first tile's pass count; a last, smaller tile may go deeper but need not

@@ -291,7 +291,6 @@ struct GemvMmaArgs {
     const uint8_t* xprep;    // activation records written by gemv_xprep_kernel (xmode < 0)
     float* partial;          // [max_slots][rows][OUT]
     unsigned long long* tile_counters;   // [col_tiles][GM_WARPS] words {marker, count}, see gemv_count_arrival
-    int* status;             // holds the call tag when a bounded wait gave up during this call
     int* sticky;             // the library's per-device status word (may be null)
     __nv_bfloat16* y;        // [M][OUT]
     float* y_f32;            // optional
@@ -310,7 +309,6 @@ struct GemvMmaArgs {
     __nv_bfloat16* h_out;
     int ldx, r_is_f32;
     float eps;
-    uint32_t tag;            // identifies this call in the counters and the status word; 31 bits, never 0
     int table_bytes;         // shared memory in front of the ring that holds the in-kernel record table
     int natural;             // in-kernel records in natural element order (see XprepArgs)
     int early;               // first ring-full of weights goes out before the wait on the kernel in front
@@ -534,7 +532,7 @@ __device__ __forceinline__ unsigned int gemv_count_arrival(const GemvMmaArgs& a,
             __nanosleep(64);
         }
         if (!ok) {
-            report_wait_failure(a.status, (int)a.tag, a.sticky, WAIT_FAIL_GEMV_MMA);
+            report_wait_failure(a.sticky, WAIT_FAIL_GEMV_MMA);
             return 0u;
         }
     }
@@ -700,7 +698,7 @@ gemv_u4gs2_mma_kernel(const GemvMmaArgs a) {
                 if (it == rel_it) chain_release();
                 if (inject && it == a.skip_stage) break;          // the consumers' wait for this stage runs out
                 if (!mbar_wait_bounded(smem_u32(&bar_empty[s]), ph, a.max_polls)) {
-                    report_wait_failure(a.status, (int)a.tag, a.sticky, WAIT_FAIL_GEMV_MMA);
+                    report_wait_failure(a.sticky, WAIT_FAIL_GEMV_MMA);
                     break;
                 }
                 ++issued;
@@ -742,7 +740,7 @@ gemv_u4gs2_mma_kernel(const GemvMmaArgs a) {
         for (int p = 0; p < PASSES; ++p) acc[q][p][0] = acc[q][p][1] = 0.0f;
     // A wait that gives up marks the warp aborted: it sets the status word, stops waiting and
     // computing, still releases its stages and still takes part in the tile hand-off, where its
-    // outputs become NaN (directly, or through the status word the finishing warp reads).
+    // sums are NaN.  Nothing of it outlives the launch: a replay in which no wait gives up is right.
     bool aborted = false;
 
     int s = 0;
@@ -752,9 +750,10 @@ gemv_u4gs2_mma_kernel(const GemvMmaArgs a) {
         if ((it == 0 || blk == 0) && lane == 0)
             marker_sh[warp] = *reinterpret_cast<volatile unsigned int*>(a.tile_counters + c * GM_WARPS + warp);
         if (!aborted && !mbar_wait_bounded(smem_u32(&bar_full[s]), ph, a.max_polls)) {
-            report_wait_failure(a.status, (int)a.tag, a.sticky, WAIT_FAIL_GEMV_MMA);
+            report_wait_failure(a.sticky, WAIT_FAIL_GEMV_MMA);
             aborted = true;
         }
+        aborted = __any_sync(0xffffffffu, aborted);                      // one decision per warp: the MMAs are warp-wide
         MSAQ_TR(1, 4, tid == 0 && it == 0);
         const int cv = min(TC, a.OUT - c * TC);
         if (!aborted) {
@@ -852,7 +851,6 @@ gemv_u4gs2_mma_kernel(const GemvMmaArgs a) {
                     arrived = __shfl_sync(0xffffffffu, arrived, 0);
                     if (arrived == (unsigned int)nslots) {
                         __threadfence();
-                        const bool poison = __ldcg(a.status) == (int)a.tag;        // a wait gave up somewhere in this call
                         uint32_t seq = 0u;
                         if constexpr (PUSH) seq = gemv_push_seq(a.push);
                         // An item is four adjacent outputs (row m, group q, quad of the warp's 16 columns); 32 / S items are
@@ -889,7 +887,6 @@ gemv_u4gs2_mma_kernel(const GemvMmaArgs a) {
                                 sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
                             }
                             if (live && part == 0) {
-                                if (poison) sum.x = sum.y = sum.z = sum.w = __int_as_float(0x7FC00000);
                                 const int64_t y0 = (int64_t)a.m0 * a.OUT + e;
                                 if constexpr (PUSH) {
                                     gemv_push(a.push, y0, sum.x, seq);

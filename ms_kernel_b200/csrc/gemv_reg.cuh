@@ -262,7 +262,6 @@ struct GemvRegArgs {
     const __nv_bfloat16* X;      // row m0 of [M][K], 16-byte aligned
     float* partial;              // [max_slots][rows][OUT]
     unsigned long long* tile_counters;
-    int* status;                 // holds the call tag when a bounded wait gave up during this call
     int* sticky;
     __nv_bfloat16* y;
     float* y_f32;                // optional
@@ -271,7 +270,6 @@ struct GemvRegArgs {
     GemvSchedule sch;            // sch.nb counts units of GR_KB K blocks
     uint32_t max_polls;
     int skip_stage;
-    uint32_t tag;
     int combine;                 // split tiles are added up by gemv_umma_combine_kernel instead of the last warp to arrive
 };
 
@@ -329,7 +327,7 @@ gemv_reg_kernel(const GemvRegArgs a) {
             while (blk >= sch.nb) { blk -= sch.nb; ++c; }
             bool stop = inject && it == a.skip_stage;
             if (!stop && !mbar_wait_bounded(smem_u32(&bar_empty[s]), ph, a.max_polls)) {
-                report_wait_failure(a.status, (int)a.tag, a.sticky, WAIT_FAIL_GEMV_MMA);
+                report_wait_failure(a.sticky, WAIT_FAIL_GEMV_MMA);
                 stop = true;
             }
             if (__any_sync(0xffffffffu, stop)) break;
@@ -388,7 +386,7 @@ gemv_reg_kernel(const GemvRegArgs a) {
             const int kleft = a.NB - (next - base) * GR_KB;                   // K blocks from here to the tile's end
             if (!aborted) aborted = !mbar_wait_bounded(smem_u32(&bar_full[s]), ph, a.max_polls);
             if (__any_sync(0xffffffffu, aborted)) {                           // one decision per warp: the MMAs are warp-wide
-                if (aborted) report_wait_failure(a.status, (int)a.tag, a.sticky, WAIT_FAIL_GEMV_MMA);
+                if (aborted) report_wait_failure(a.sticky, WAIT_FAIL_GEMV_MMA);
                 aborted = true;
             } else {
                 const uint32_t so = s * STAGE;
@@ -471,13 +469,12 @@ gemv_reg_kernel(const GemvRegArgs a) {
             if (nq > 0 && nslots > 1 && !a.combine) {
                 __syncwarp();
                 GemvMmaArgs h{};                                              // the hand-off's part of the arguments
-                h.status = a.status; h.sticky = a.sticky; h.max_polls = a.max_polls; h.tag = a.tag;
+                h.sticky = a.sticky; h.max_polls = a.max_polls;
                 unsigned int arrived = 0;
                 if (lane == 0) arrived = gemv_count_arrival(h, a.tile_counters + c * GM_WARPS + cw, marker_sh[cw]);
                 arrived = __shfl_sync(0xffffffffu, arrived, 0);
                 if (arrived == (unsigned int)nslots) {
                     __threadfence();
-                    const bool poison = __ldcg(a.status) == (int)a.tag;       // a wait gave up somewhere in this call
                     // four adjacent outputs per item, S lanes to an item where there are few (see gemv_mma.cuh): the order
                     // of the additions depends on the shape alone
                     const int64_t sstride4 = (int64_t)a.rows * a.OUT / 4;
@@ -509,7 +506,6 @@ gemv_reg_kernel(const GemvRegArgs a) {
                             sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
                         }
                         if (live && part == 0) {
-                            if (poison) sum.x = sum.y = sum.z = sum.w = nan;
                             const int64_t y0 = (int64_t)a.m0 * a.OUT + e;
                             if (a.y_f32) *reinterpret_cast<float4*>(a.y_f32 + y0) = sum;
                             if (MT == 1 && a.res) {        // the projection rounds to bf16 first, as the unfused add sees it

@@ -535,11 +535,11 @@ gemv_umma_kernel(const GemvUmmaArgs a) {
 
 // Sum of the split-K partials of the tensor-memory kernel, in slot order: one thread per four
 // consecutive outputs of one activation row.  Tiles that one CTA covered alone were written by
-// that CTA and are skipped.  A status word that says that a wait gave up marks the whole launch NaN: the tensor-memory
-// kernel clears the word in front (tag == 0: any value counts), the register kernel leaves its call's tag there.
+// that CTA and are skipped.  A status word that says that a wait gave up marks the whole launch NaN (the staging kernel clears it);
+// null for the register kernel, whose partial sums are NaN themselves then.
 __global__ void __launch_bounds__(256)
 gemv_umma_combine_kernel(const float* __restrict__ partial, const int* __restrict__ status, __nv_bfloat16* __restrict__ y,
-                         float* __restrict__ y_f32, GemvSchedule sch, int m0, int rows, int OUT, int tag) {
+                         float* __restrict__ y_f32, GemvSchedule sch, int m0, int rows, int OUT) {
     chain_release();
     chain_wait();
     const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -547,7 +547,7 @@ gemv_umma_combine_kernel(const float* __restrict__ partial, const int* __restric
     if (idx >= (int64_t)rows * quads) return;
     const int m = (int)(idx / quads), col = (int)(idx % quads) * 4, c = col / sch.tc;
     const int first = sch.first_cta(c), nslots = sch.last_cta(c) - first + 1;
-    const bool poison = tag ? *status == tag : *status != 0;
+    const bool poison = status && *status != 0;
     if (nslots == 1 && !poison) return;
     const int64_t sstride = (int64_t)rows * OUT;
     const float* src = partial + (int64_t)m * OUT + col;

@@ -69,9 +69,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // OR `bit` into the library's sticky per-device word that msaq_wait_status() reports to the host.
 constexpr int WAIT_FAIL_GEMV_MMA = 1, WAIT_FAIL_GEMV_UMMA = 2, WAIT_FAIL_KV_DECODE = 4, BAD_APPEND_POS = 8,
               PEER_EXCHANGE_TIMEOUT = 16;
+__device__ __forceinline__ void report_wait_failure(int* sticky, int bit) {
+    if (sticky) atomicOr(sticky, bit);
+}
+// for the kernels whose outputs are marked through a word of the call's workspace, which the launch in front of them clears
 __device__ __forceinline__ void report_wait_failure(int* status, int value, int* sticky, int bit) {
     atomicExch(status, value);
-    if (sticky) atomicOr(sticky, bit);
+    report_wait_failure(sticky, bit);
 }
 
 // TMA bulk copy global -> shared of `bytes` (multiple of 16, both addresses

@@ -69,6 +69,52 @@ def test_gemv_wait_gives_up_and_next_call_is_correct(rng, M):
     assert _status() == 0
 
 
+@pytest.mark.parametrize("u,M", [(4, 1), (4, 4), (4, 6), (4, 12), (3, 2)])
+def test_replay_does_not_depend_on_an_earlier_give_up(rng, u, M):
+    """What a call that gave up leaves in the workspace must not reach a captured call that waits for nothing: the first word,
+    where such a call used to leave its number, may hold anything.  More columns than one wave of the direct kernels, split
+    tiles, each of the kernels that add partial sums up."""
+    import cabi
+    from ms_kernel_b200 import _lib
+    L = _lib.lib()
+    OUT, K = 10256, 1056
+    W = orc.to_bf16((rng.standard_normal((OUT, K)) * 0.02).astype(np.float32))
+    X = orc.to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    p = orc.pack_weight(W, u, 2)
+    pd = cabi.planes_to_dev(p)
+    ref = orc.wonly_matmul(p, X)
+    x = cabi.bf16_dev(X)
+    y = torch.zeros((M, OUT), dtype=torch.bfloat16, device="cuda")
+    yf = torch.zeros((M, OUT), dtype=torch.float32, device="cuda")
+    wsb = L.msaq_wonly_gemv_workspace(M, OUT, K // 32, u, 2)
+    ws = torch.zeros(wsb, dtype=torch.uint8, device="cuda")
+    word = ws[:4].view(torch.int32)
+
+    def call(stream):
+        _lib.check(L.msaq_wonly_gemv_batched(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
+                                             pd["shared_cm"].data_ptr(), y.data_ptr(), yf.data_ptr(), M, OUT, K // 32, u, 2,
+                                             ws.data_ptr(), wsb, stream.cuda_stream))
+    _status()
+    with _short_waits(0):
+        call(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+    assert _status() & 1 and torch.isnan(yf).any()
+    left = int(word.item())
+    g = torch.cuda.CUDAGraph()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(g, stream=s):
+        call(s)
+    torch.cuda.synchronize()
+    for value in (left, left + 1, left + 2, -1):
+        word.fill_(value)
+        yf.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        cabi.check_output(y.float().cpu().numpy(), yf.cpu().numpy(), ref, MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+    assert _status() == 0
+
+
 def test_decode_wait_gives_up_and_next_call_is_correct(rng):
     import cabi
     u, gs, Hq, Hkv, Lk, D = 4, 2, 8, 2, 512, 128
