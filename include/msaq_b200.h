@@ -125,9 +125,9 @@ int msaq_wonly_gemv_wide(const void* x, const int8_t* scale_exp, const uint8_t* 
 
 /*
  * Y[M,OUT] = X[M,K] . dequant(W)^T on column-major planes, any M >= 1.
- * (The tensor-memory kernel -- gs = 2, more than 32 rows -- widens q * 2^e through an
- * fp32 constant of about 2^23 * 2^e: block exponents above 104 overflow there.  bf16 weights of magnitude below
- * 2^110 never produce them.)
+ * (The tensor-memory kernel widens q * 2^e through an fp32 constant of about 2^23 * 2^e: block exponents above 104 overflow
+ * there.  bf16 weights of magnitude below 2^110 never produce them.  It serves gs = 2 from 33 rows on, and fewer rows -- u = 4
+ * from nine, u = 2 and 3 from one -- where X is not 16-byte aligned or the workspace is smaller than the query says.)
  * Replaces op `msaq::wonly_gemv_batched` (csrc/pybind.cpp:205-206, host
  * csrc/w_gemv.cu:1514-1570).
  */

@@ -102,3 +102,18 @@ def test_non_finite_activation_gives_a_nan_row(rng, bad, M, OUT, K):
     X[M - 2, K - 3] = bad
     _, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
     assert np.isnan(gotf[M - 2]).all() and np.isfinite(np.delete(gotf, M - 2, 0)).all()
+
+
+@pytest.mark.parametrize("u,M", [(4, 3), (4, 5), (4, 8), (4, 9), (3, 1), (3, 12), (2, 6), (2, 30)])
+@pytest.mark.parametrize("OUT,K", [(256, 96), (9616, 96)])
+def test_largest_finite_weights(rng, u, M, OUT, K):
+    """Weights of 2^127 and more (block exponent 121, the largest that finite values give), direct and register kernels."""
+    import cabi
+    W = rng.standard_normal((OUT, K)) * 0.05
+    huge = np.sign(W[::3, :32]) * 2.0 ** 127 * rng.uniform(1.0, 1.99, W[::3, :32].shape)
+    W[::3, :32] = huge * (rng.random(huge.shape) < 0.7)
+    X = orc.to_bf16(rng.standard_normal((M, K)).astype(np.float32) * np.float32(2.0 ** -60))
+    p = orc.pack_weight(orc.to_bf16(W.astype(np.float32)), u, 2)
+    assert p["scale_exp"].max() == 121
+    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    cabi.check_output(got, gotf, orc.wonly_matmul(p, X), MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
