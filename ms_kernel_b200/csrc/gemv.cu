@@ -226,13 +226,24 @@ struct RegPlan {
     size_t partial_off, total;
 };
 
-// Whether the register kernel is the one for these sizes (where the direct kernels are not).  u = 4 from five to eight rows:
-// up to about 100 MB (8192x8192, eight rows: 31.3 us on the integer kernel, 24.6; 28672x4096: 36.4, 33.4; 57344x8192, 367 MB:
-// 95.4, 110.4).  From 33 rows on up to about 48 MB (64 rows against the tensor-memory kernel: 6144x4096 41.3 -> 25.6,
-// 4096x14336, 46 MB, 48.2 -> 44.5, 8192x8192, 52 MB, 46.8 -> 47.8, 28672x4096 67.9 -> 80.5).
+// Whether the register kernel is the one for these sizes (where the direct kernels are not).
+//   u = 4, five to eight rows: up to about 100 MB (8192x8192, eight rows: 32.0 us on the integer kernel, 23.5; 28672x4096: 35.6, 33.0;
+//     57344x8192, 367 MB: 93.4, 110.4).
+//   17 to 32 rows: all, but for u = 3 the very largest (32 rows, tensor-memory kernel -> this one: 28672x4096 61.3 -> 59.0, 57344x8192,
+//     396 MB, 183.0 -> 185.3; u = 4 163.6 -> 157.6).
+//   33 to 64 rows: the MMAs of eight n-tiles cost the same whether they are full or not and grow with the number of weights, the
+//     tensor-memory kernel's time grows with the rows; many columns suit that kernel.  u4, 33 | 48 | 64 rows, us there -> here:
+//     6144x4096 31.8 -> 24.8 | 34.3 -> 25.2 | 40.1 -> 25.8     5120x8192 37.6 -> 33.9 | 43.0 -> 34.4 | 47.1 -> 35.1
+//     14336x3072 33.1 -> 35.7 | 37.7 -> 36.6 | 42.4 -> 37.8    4096x14336 41.8 -> 43.9 | 44.3 -> 44.5 | 48.6 -> 44.8
+//     14336x4096 37.8 -> 43.3 | 42.4 -> 44.5 | 47.1 -> 45.7    57344x512 31.9 -> 33.3 | 36.9 -> 35.1 | 43.3 -> 37.4
+//     u3 at 64 rows: 12288x4096, 42 MB, 49.2 -> 44.2, 14336x4096, 50 MB, 49.2 -> 50.2.
 bool reg_serves(int64_t M, int64_t OUT, int64_t NB, int u) {
     const int64_t bytes = OUT * NB * (gr_ub(u) + gr_sb(u) + 1);
-    if (M > GR_MAX_M || (M > 32 && bytes > (48LL << 20))) return false;
+    if (M > GR_MAX_M || (M > 16 && u == 3 && bytes > (300LL << 20))) return false;
+    if (M > 32) {
+        if (bytes > (u == 3 ? 45LL << 20 : 48LL << 20)) return false;
+        if (M <= 48 && OUT * (NB * BLOCK + 1000) > (M <= 40 ? 57000000 : 66000000)) return false;
+    }
     return u != 4 || M >= GU_MIN_M || (M >= 5 && bytes <= (100LL << 20));
 }
 

@@ -117,3 +117,24 @@ def test_largest_finite_weights(rng, u, M, OUT, K):
     assert p["scale_exp"].max() == 121
     got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
     cabi.check_output(got, gotf, orc.wonly_matmul(p, X), MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
+
+
+@pytest.mark.parametrize("u,M,OUT,K,launches", [(4, 33, 6144, 4096, 2), (4, 33, 4096, 11008, 2), (4, 33, 14336, 3072, 3), (4, 40, 4096, 14336, 3),
+                                                (4, 48, 14336, 3072, 2), (4, 48, 14336, 4096, 3), (4, 49, 14336, 4096, 2), (4, 64, 4096, 14336, 2),
+                                                (3, 64, 12288, 4096, 2), (3, 64, 14336, 4096, 3), (2, 36, 57344, 512, 3), (2, 17, 57344, 512, 2)])
+def test_row_counts_where_the_kernels_take_turns(u, M, OUT, K, launches):
+    """On either side of each line between this kernel (itself and the sum of its partials) and the tensor-memory kernel
+    (staging, itself, the sum), where their times cross; the two agree to the rounding of the sums."""
+    from ms_kernel_b200 import _lib, ops, pack
+    g = torch.Generator(device="cuda").manual_seed(M + OUT)
+    W = (torch.randn((OUT, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    lin = ops.PackedLinear(pack.pack_weight(W, u, 2), "cuda")
+    buf = torch.randn(M * K + 1, generator=g, device="cuda").to(torch.bfloat16)
+    x = buf[:M * K].reshape(M, K)
+    n0 = _lib.lib().msaq_launch_count()
+    y = lin.fwd(x)
+    assert _lib.lib().msaq_launch_count() - n0 == launches
+    off = torch.empty_like(buf)[1:].reshape(M, K)            # off a 16-byte boundary: always the tensor-memory kernel
+    off.copy_(x)
+    want = lin.fwd(off)
+    assert float((y.float() - want.float()).norm() / want.float().norm()) < 2e-3
