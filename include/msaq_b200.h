@@ -66,8 +66,8 @@ unsigned long long msaq_launch_count(void);
  *   the first thread block of the pipelined GEMV / flash-decode kernels stops before this pipeline stage, so
  *   that the wait for it runs out.  Used to check the give-up path without faulting or hanging anything.
  * MSAQ_OPT_EARLY_WEIGHTS (default 0): the integer-MMA GEMVs start fetching their packed weights BEFORE they wait
- *   for the kernel in front of them in the stream (only the activations wait), and every kernel of the library
- *   asks for the largest shared-memory split so that a GEMV's thread blocks can take their places on an SM while a
+ *   for the kernel in front of them in the stream (only the activations wait), as do the direct kernels of the smaller
+ *   matrices, and every kernel of the library but those asks for the largest shared-memory split so that a GEMV's thread blocks can take their places on an SM while a
  *   small kernel in front still runs there.  The contract that makes this safe is the caller's: set it only
  *   where the weight planes are complete before the GEMV is enqueued -- packed at load time and synchronised
  *   since, the serving case -- never where a kernel still in flight on the stream writes them.  Three quarters

@@ -73,18 +73,20 @@ int* sticky_status();         // device address of the per-device status word on
 // chain_wait / chain_release): every kernel of this library executes chain_wait() before it
 // touches memory another kernel produces or consumes.
 // An SM holds thread blocks of two kernels at once only under one split of its L1 / shared memory.  The streaming
-// kernels need the largest shared-memory share, so with MSAQ_OPT_EARLY_WEIGHTS every kernel of the chain asks for
-// it: otherwise the blocks of a GEMV launched early behind a small kernel (activation staging, cache append,
+// kernels need the largest shared-memory share, so with MSAQ_OPT_EARLY_WEIGHTS every kernel of the chain but the direct GEMVs
+// (launch_chained_cluster) asks for it: otherwise the blocks of a GEMV launched early behind a small kernel (activation staging, cache append,
 // residual add) could not start -- and begin fetching their weights -- until the small kernel had left every SM
 // (measured with per-block time stamps: without it the GEMV's first block starts when the staging kernel's last
 // block exits; with it 0.9 us after the staging kernel starts).
 void prefer_max_shared(const void* kernel);      // once per (kernel, device), only while the option is on
 
-// The same in clusters of `cluster` thread blocks (1: none).
+// Launches in clusters of `cluster` thread blocks (1: none) with the split of L1 and shared memory that the kernel gets by itself: the
+// direct GEMVs load their weights through L1, and under the largest shared-memory split its remainder is too small for the
+// loads in flight (MSAQ_OPT_EARLY_WEIGHTS on, us, largest split -> own split: 4096x14336 u4 one row 18.7 -> 14.5, u2 eight rows 34.5 ->
+// 22.0, 7168x8192 u4 one row 20.5 -> 14.6, where the kernel in its place before took 17.6; layer steps 8B 79.4 -> 76.0, 70B 165.1 -> 163.9).
 template <typename... P, typename... A>
 inline cudaError_t launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, cudaStream_t st,
                                           A&&... args) {
-    prefer_max_shared(reinterpret_cast<const void*>(kernel));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -107,8 +109,10 @@ inline cudaError_t launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Ordinary launches of the chain.
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    prefer_max_shared(reinterpret_cast<const void*>(kernel));
     return launch_chained_cluster(kernel, grid, block, smem, 1, st, std::forward<A>(args)...);
 }
 

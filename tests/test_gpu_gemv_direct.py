@@ -97,3 +97,42 @@ def test_back_to_back_and_replayed(rng):
         assert torch.equal(step(), want)
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("u,M,OUT,K", [(2, 8, 4096, 14336), (4, 1, 4096, 14336)])
+def test_early_weights_do_not_slow_the_kernel_down(u, M, OUT, K):
+    """The kernels load through L1, which the largest shared-memory split of the other kernels would leave too little of: 1.3 to
+    1.6 times the time before they kept their own split.  Six matrices in turn, more than L2 holds, in a replayed graph."""
+    from ms_kernel_b200 import _lib, ops
+    L = _lib.lib()
+    nb = K // 32
+    b = lambda *s: torch.randint(0, 256, s, dtype=torch.uint8, device="cuda")       # noqa: E731
+    lins = [ops.PackedLinear(dict(OUT=OUT, nb=nb, u=u, gs=2, scale_exp=torch.full((nb, OUT), -12, dtype=torch.int8, device="cuda"),
+                                  upper_cm=b(nb, OUT, 4 * (8 - u)), shared_cm=b(nb, OUT, 2 * u)), "cuda") for _ in range(6)]
+    x = torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    us = {}
+    for early in (0, 1):
+        torch.cuda.synchronize()
+        assert L.msaq_set_option(6, early) == 0
+        try:
+            s = torch.cuda.Stream()
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                lins[0].fwd(x)
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                for lin in lins * 3:
+                    lin.fwd(x)
+        finally:
+            L.msaq_set_option(6, 0)
+        times = []
+        for _ in range(12):
+            a, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.replay()
+            e.record()
+            e.synchronize()
+            times.append(a.elapsed_time(e))
+        us[early] = min(times)
+    assert us[1] < 1.15 * us[0], us
