@@ -322,18 +322,41 @@ int launch_xprep(const XprepArgs& xa, int mode, unsigned grid, cudaStream_t st) 
 }
 
 // ---- no partial sums in global memory: matrices of one wave (gemv_direct_pick), up to a size -------
-// The limits are where the pipelined kernels overtake (us per call, pipelined -> direct):
-//   u4, 1-2 rows   4096x4096 10.5 -> 6.8   8192x8192 19.3 -> 14.4   4096x28672 (92 MB) 30.0 -> 24.4   1024x8192 14.4 -> 5.8
-//   u4, 3-4 rows   4096x4096 12.1 -> 7.8   8192x8192 25.2 -> 20.0   8192x14336 (92 MB) 33.1 -> 32.3, 4096x28672 31.7 -> 33.8
-//   u4, 5-8 rows   4096x4096 16.7 -> 7.9   8192x8192 31.0 -> 22.0   4096x28672 38.3 -> 37.8
-//   u4, 9-16 rows  4096x4096 13.9 -> 8.5   4096x14336 (46 MB) 25.8 -> 22.0   8192x8192 (52 MB) 25.7 -> 26.7
-//   u3             4096x4096 14.1 -> 8.8   4096x14336, 8 rows 26.9 -> 22.8, 16 rows 28.8 -> 30.7
-//   u2             4096x4096 13.6 -> 8.0   4096x14336 (53 MB), 8 rows 25.6 -> 21.5, 16 rows 27.6 -> 23.4
+// The limits are where the pipelined kernels overtake (us per call, pipelined -> direct, matrices in turn so that none is in L2):
+//   u4, 1 row      4096x4096 10.9 -> 6.8   8192x8192 19.9 -> 15.0   4096x28672 (92 MB) 30.0 -> 24.3   1024x8192 14.9 -> 5.8
+//   u4, 4 rows     4096x4096 12.8 -> 8.4   8192x8192 23.9 -> 20.5   5120x14336 (57 MB) 24.3 -> 32.5
+//   u4, 5-8 rows   4096x4096 14.4 -> 7.7   8192x8192 23.5 -> 22.2   4096x28672 34.3 -> 36.7
+//   u4, 9-16 rows  4096x4096 14.4 -> 8.6   4096x14336 (46 MB) 25.8 -> 22.2   8192x8192 (52 MB) 26.1 -> 27.3
+//   u3             4096x4096 15.0 -> 9.0   4096x14336, 8 rows 27.4 -> 23.5, 16 rows 29.3 -> 31.4
+//   u2             4096x4096 14.9 -> 8.2   4096x14336 (53 MB), 8 rows 26.5 -> 21.9, 16 rows 28.0 -> 24.1
+// Below the limits the integer kernel is still the slower one where the thread blocks leave SMs idle and K is long (5120 columns are
+// 80 thread blocks, and 80 clusters of two do not fit), the more so with a prologue, which every thread block evaluates over the
+// whole of K.  So the model's cycles are held against what the pipelined kernel's time grows with: the bytes, and K where the
+// staging kernel adds and takes a norm.  Matrices so narrow that that kernel's tiles are at their narrowest never cross below the
+// limits.  us, pipelined -> direct:
+//   plain     3 rows   4096x14336 22.0 -> 19.3   5120x14336 24.4 -> 32.0
+//   silu      1 row    4096x14336 20.7 -> 15.3   5120x14336 23.2 -> 24.1
+//             3 rows   4096x4096 13.6 -> 10.9    8192x4096 18.4 -> 16.6   4096x14336 22.5 -> 28.3   5120x14336 24.0 -> 49.6
+//   add+norm  2 rows   4096x14336 27.8 -> 23.0   5120x11008 23.8 -> 29.8
+bool direct_int_pays(int mode, int64_t M, int64_t OUT, int64_t NB, int64_t cycles) {
+    if ((OUT + 2 * GM_GROUP - 1) / (2 * GM_GROUP) * 32 < GM_CTAS_PER_SM * sm_count()) return true;
+    struct Line { int base, per_mb, per_krow; };
+    constexpr int ALWAYS = 1 << 30;
+    static const Line norm[4] = {{ALWAYS, 0, 0}, {16000, 400, 0}, {13000, 400, 0}, {12000, 600, 0}};        // and plain
+    static const Line silu[4] = {{7000, 400, 0}, {12000, 300, 0}, {7000, 300, 0}, {10000, 300, 0}};
+    static const Line add_norm[4] = {{ALWAYS, 0, 0}, {8000, 200, 400}, {10000, 100, 400}, {9000, 200, 400}};
+    const Line& l = (mode == XP_SILU_MUL ? silu : mode == XP_ADD_NORM ? add_norm : norm)[M - 1];
+    const int64_t bytes = OUT * NB * gm_col_bytes(GF_MSAQ_U4);
+    return cycles <= l.base + bytes * l.per_mb / 1000000 + M * NB * BLOCK * l.per_krow / 1000;
+}
+
 // The test hook stops a copy-issuing thread: it belongs to the pipelined kernels, which run while it is set.
 bool direct_usable(const void* X, int mode, int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs) {
     if (M > (mode == XP_PLAIN ? GD_MAX_M : 4) || option_test_skip_stage() >= 0 || (reinterpret_cast<uintptr_t>(X) & 15)) return false;
     const int64_t limit = u == 4 ? (M <= 2 ? 100 : M <= 8 ? 60 : 48) : u == 2 || M <= 8 ? 60 : 24;
-    return OUT * NB * (gr_ub(u) + gr_sb(u) + 1) <= (limit << 20) && gemv_direct_pick(M, OUT, NB, u, cg, cs);
+    int64_t cycles = 0;
+    return OUT * NB * (gr_ub(u) + gr_sb(u) + 1) <= (limit << 20) && gemv_direct_pick(M, OUT, NB, u, cg, cs, &cycles) &&
+           (u != 4 || M > 4 || direct_int_pays(mode, M, OUT, NB, cycles));
 }
 
 int run_direct(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh, void* Y,

@@ -46,7 +46,7 @@ bool integer(int64_t M, int u) { return u == 4 && M <= 4; }
 // 2048: 3.5 against 4.9).  Clusters that do not fit the GPCs wait for a second round (1216 x 18688,
 // 19 clusters of seven: 14.6 us, 76 of three: 11.1 us; the occupancy query counts 148, 74, 45, 33, 26, 22, 15 and 15 clusters of one
 // to eight thread blocks, one to an SM; GPCs differ by a few SMs from part to part, hence a little less here).
-bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs) {
+bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs, int64_t* cycles) {
     static const int int1[] = {1, 4, 0}, int4[] = {2, 4, 0}, bf4[] = {2, 3, 4, 0}, bf3[] = {2, 3, 0};
     const int* widths = integer(M, u) ? (M == 1 ? int1 : int4) : u == 4 ? bf4 : bf3;
     const int64_t stage = integer(M, u) ? 55 * M : 20, group = integer(M, u) ? 45 : (u == 4 ? 95 : u == 3 ? 115 : 105) + (M > 8 ? 15 : 0);
@@ -67,6 +67,7 @@ bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* c
             }
         }
     }
+    *cycles = best;
     return best != INT64_MAX;
 }
 

@@ -465,8 +465,9 @@ gemv_direct_bf16_kernel(const GemvDirectArgs a) {
     gd_finish<ROWS, COLS, WARPS>(a, red, part, c0);
 }
 
-// gemv_direct.cu.  Column groups per thread block and thread blocks per cluster for these sizes; false: not one wave.
-bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs);
+// gemv_direct.cu.  Column groups per thread block and thread blocks per cluster for these sizes, and the model's cycles; false:
+// not one wave.
+bool gemv_direct_pick(int64_t M, int64_t OUT, int64_t NB, int u, int* cg, int* cs, int64_t* cycles);
 int gemv_direct_launch(const GemvDirectArgs& a, int u, int mode, int cg, cudaStream_t st);
 
 }  // namespace msaq

@@ -136,3 +136,31 @@ def test_early_weights_do_not_slow_the_kernel_down(u, M, OUT, K):
             times.append(a.elapsed_time(e))
         us[early] = min(times)
     assert us[1] < 1.15 * us[0], us
+
+
+@pytest.mark.parametrize("mode,M,OUT,K,launches", [(0, 1, 7168, 8192, 1), (0, 3, 4096, 14336, 1), (0, 3, 5120, 14336, 2), (0, 4, 5120, 11008, 2),
+                                                   (1, 1, 5120, 14336, 1), (1, 4, 5120, 11008, 2), (2, 1, 4096, 14336, 1),
+                                                   (2, 1, 5120, 14336, 2), (2, 2, 8192, 8192, 2), (2, 3, 4096, 4096, 1), (2, 3, 5120, 14336, 2),
+                                                   (2, 4, 2048, 28672, 1), (3, 1, 4096, 14336, 1), (3, 2, 5120, 11008, 2)])
+def test_where_the_integer_kernel_and_the_pipelined_one_take_turns(mode, M, OUT, K, launches):
+    """u = 4, up to four rows, on either side of the lines where their times cross: this kernel alone, or the staging kernel and
+    the pipelined one.  Either gives what the pipelined kernel gives, to the rounding of the sums."""
+    from ms_kernel_b200 import _lib, ops, pack
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M + OUT + K)
+    lin = ops.PackedLinear(pack.pack_weight((torch.randn((OUT, K), generator=g, device="cuda") * 0.02).to(torch.bfloat16), 4, 2), "cuda")
+    x = torch.randn((M, (2 if mode == 2 else 1) * K), generator=g, device="cuda").to(torch.bfloat16)
+    d = torch.randn((M, K), generator=g, device="cuda") if mode == 3 else None
+
+    def call():
+        n0 = L.msaq_launch_count()
+        y = lin.fwd(x) if mode == 0 else lin.fwd_fused(x, mode, d)
+        return y[0] if mode == 3 else y, L.msaq_launch_count() - n0
+    y, n = call()
+    assert n == launches
+    assert L.msaq_set_option(4, 1 << 30) == 0            # the hook's stage is never reached: the pipelined kernel, undisturbed
+    try:
+        want, n = call()
+    finally:
+        L.msaq_set_option(4, -1)
+    assert n == 2 and orc.rel_fro(y.float().cpu().numpy(), want.float().cpu().numpy()) < REL_FRO_TOL
