@@ -79,10 +79,10 @@ __device__ __forceinline__ GrLane gr_lane(int t) {
 // Eight weights of one row as bf16 pairs: w[j] = elements (8t + j, 8t + j + 4) of the 32-block.
 //
 // q = up * 2^u + sh.  A code with its sign bit flipped, dropped into the mantissa of bf16 128.0, reads as 128 + 2^(b-1) + code
-// (b its width).  up * 2^u and sh come out of one fused multiply-add each, sh * 2^e and then q * 2^e of another; every value on the
-// way is an integer of at most eight significant bits times a power of two, so nothing is rounded, and none is larger than
-// the largest code times 2^e: the whole range of block exponents that finite weights have (up to 121) is served.  (With the scale
-// inside the offset, -(128 + 2^(u-1)) * 2^e, weights of 2^127 and more came out as Inf or NaN; as many instructions.)
+// (b its width).  h = (sh + 64) * 2^e and then h + (up - 64 / 2^u) * 2^(u+e) are formed with one fused multiply-add each; every
+// value on the way is an integer of at most eight significant bits times a power of two, so nothing is rounded.  The 64 that goes
+// from one part to the other keeps the offsets, -(64 + 2^(u-1)) * 2^e among them, inside bf16 over the whole range of block
+// exponents that finite weights have (up to 121; with -(128 + 2^(u-1)) * 2^e weights of 2^127 and more came out as Inf or NaN).
 // The constants of the decode below, read back from shared memory once: as literals they are put into registers again at
 // every use (LOP3 and HFMA2 take one immediate at most), which doubles the instructions of a step.
 template <int U>
@@ -96,8 +96,8 @@ struct GrConst {
             case 1: return 0x43004300u | (0x00010001u << (WB - 1));                  // bf16 128.0, and the code's sign bit
             case 2: return ((1u << U) - 1u) * 0x00010001u;
             case 3: return 0x43004300u | (0x00010001u << (U - 1));
-            case 4: return ((WB == 4 ? 0xC308u : WB == 5 ? 0xC310u : 0xC320u) + (U << 7)) * 0x00010001u;   // -(128 + 2^(WB-1)) * 2^U
-            case 5: return (U == 4 ? 0xC308u : U == 3 ? 0xC304u : 0xC302u) * 0x00010001u;     // -(128 + 2^(U-1))
+            case 4: return (U == 4 ? 0xC30Cu : U == 3 ? 0xC318u : 0xC330u) * 0x00010001u;     // -(128 + 2^(WB-1) + 64 / 2^U)
+            case 5: return (U == 4 ? 0xC290u : U == 3 ? 0xC288u : 0xC284u) * 0x00010001u;     // -(64 + 2^(U-1))
             case 6: return ((127u + U) << 7) * 0x00010001u;                          // 2^U
             case 7: return 0x3F803F80u;
             default: return 0x80008000u;                                             // -0: the neutral addend
@@ -120,6 +120,8 @@ template <int U>
 __device__ __forceinline__ void gr_decode(const GrRaw& in, const GrLane& ln, const GrConst<U>& k, uint32_t (&w)[4]) {
     constexpr int WB = 8 - U;
     const uint32_t s = (uint32_t)(in.e * 0x00800080 + 0x3F803F80);                    // 2^e twice
+    const uint32_t su = hfma2_bf16(s, k.two_u, k.neg0), ns = hfma2_bf16(s, k.soff, k.neg0);
+
     uint32_t f[4];                       // upper codes j (low half) and j + 4 (high half), other bits arbitrary
     if constexpr (U == 4) {
         f[0] = in.w0; f[1] = in.w0 >> 4; f[2] = in.w0 >> 8; f[3] = in.w0 >> 12;
@@ -144,10 +146,9 @@ __device__ __forceinline__ void gr_decode(const GrRaw& in, const GrLane& ln, con
         const uint32_t v = prmt(in.s0, in.s1, 0x5410u) >> ln.sh_shift & 0xFFFu;
         g = v | (v << 10);
     } else g = in.s0 | (in.s0 << 12);
-    const uint32_t h0 = hfma2_bf16(hfma2_bf16(and_xor(g, k.sm, k.sx), k.one, k.soff), s, k.neg0);
-    const uint32_t h1 = hfma2_bf16(hfma2_bf16(and_xor(g >> U, k.sm, k.sx), k.one, k.soff), s, k.neg0);
+    const uint32_t h0 = hfma2_bf16(and_xor(g, k.sm, k.sx), s, ns), h1 = hfma2_bf16(and_xor(g >> U, k.sm, k.sx), s, ns);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) w[j] = hfma2_bf16(hfma2_bf16(and_xor(f[j], k.um, k.ux), k.two_u, k.uoff), s, j < 2 ? h0 : h1);
+    for (int j = 0; j < 4; ++j) w[j] = hfma2_bf16(hfma2_bf16(and_xor(f[j], k.um, k.ux), k.one, k.uoff), su, j < 2 ? h0 : h1);
 }
 
 // The same from shared memory: ub, sb, eb are the addresses of this lane's codes and of the row's scale, OFF* constant
