@@ -120,8 +120,10 @@ def test_largest_finite_weights(rng, u, M, OUT, K):
 
 
 @pytest.mark.parametrize("u,M,OUT,K,launches", [(4, 33, 6144, 4096, 2), (4, 33, 4096, 11008, 2), (4, 33, 14336, 3072, 3), (4, 40, 4096, 14336, 3),
-                                                (4, 48, 14336, 3072, 2), (4, 48, 14336, 4096, 3), (4, 49, 14336, 4096, 2), (4, 64, 4096, 14336, 2),
-                                                (3, 64, 12288, 4096, 2), (3, 64, 14336, 4096, 3), (2, 36, 57344, 512, 3), (2, 17, 57344, 512, 2)])
+                                                (4, 44, 14336, 2048, 2), (4, 48, 4096, 14336, 2), (4, 48, 14336, 3072, 3), (4, 49, 14336, 4096, 3),
+                                                (4, 64, 14336, 4096, 2), (4, 64, 57344, 512, 2), (3, 37, 47056, 256, 2), (3, 54, 42272, 1088, 3),
+                                                (3, 64, 12288, 4096, 2), (3, 64, 14336, 4096, 3), (2, 36, 57344, 512, 2), (2, 36, 28672, 1536, 3),
+                                                (2, 17, 57344, 512, 2)])
 def test_row_counts_where_the_kernels_take_turns(u, M, OUT, K, launches):
     """On either side of each line between this kernel (itself and the sum of its partials) and the tensor-memory kernel
     (staging, itself, the sum), where their times cross; the two agree to the rounding of the sums."""
