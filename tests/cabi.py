@@ -28,9 +28,41 @@ def bf16_dev(a):
     return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to(torch.bfloat16).cuda()
 
 
-def gemv(kind, x, p, M=1, want_f32=True):
-    """kind in {'rowmajor','wide','batched'}; x bf16 device tensor; p dict of device planes.
-    Returns (y bf16 as float32 numpy, y_f32 numpy or None)."""
+class options:
+    """The library's options {number: value} for the duration of a with block."""
+
+    def __init__(self, values):
+        self.values = values
+
+    def __enter__(self):
+        L = _lib.lib()
+        self.before = {k: L.msaq_get_option(k) for k in self.values}
+        for k, v in self.values.items():
+            assert L.msaq_set_option(k, v) == 0
+
+    def __exit__(self, *a):
+        for k, v in self.before.items():
+            _lib.lib().msaq_set_option(k, v)
+
+
+def pipelined():
+    """Matrices of one wave on the pipelined kernels instead of the direct ones, which have no use for the hook that stops a
+    copy-issuing thread and stay out while it is set.  No launch reaches this stage, so nothing is stopped."""
+    return options({4: 1 << 30})
+
+
+def off_16(x):
+    """A copy of x (bf16) that starts two bytes past a 16-byte boundary: the GEMVs from nine rows on (u = 2, 3: all) then run on
+    the tensor-memory kernel, whatever their size."""
+    buf = torch.empty(x.numel() + 1, dtype=torch.bfloat16, device="cuda")
+    buf[1:] = x.reshape(-1)
+    assert buf.data_ptr() % 16 == 0
+    return buf[1:]
+
+
+def gemv(kind, x, p, M=1, want_f32=True, fill=None):
+    """kind in {'rowmajor','wide','batched'}; x bf16 device tensor; p dict of device planes; `fill`: what the bytes of the
+    workspace hold before the call.  Returns (y bf16 as float32 numpy, y_f32 numpy or None)."""
     L = _lib.lib()
     OUT, NB, u, gs = int(p["OUT"]), int(p["nb"]), int(p["u"]), int(p["gs"])
     shape = (OUT,) if kind != "batched" else (M, OUT)
@@ -38,6 +70,8 @@ def gemv(kind, x, p, M=1, want_f32=True):
     yf = torch.empty(shape, dtype=torch.float32, device="cuda") if want_f32 else None
     wsb = L.msaq_wonly_gemv_workspace(M, OUT, NB, u, gs)
     ws = torch.empty(max(wsb, 256), dtype=torch.uint8, device="cuda")
+    if fill is not None:
+        ws.fill_(fill)
     if kind == "rowmajor":
         rc = L.msaq_wonly_gemv(_ptr(x), _ptr(p["scale_exp"]), _ptr(p["upper"]), _ptr(p["shared"]), _ptr(y), _ptr(yf),
                                OUT, NB, u, gs, _ptr(ws), wsb, _stream())

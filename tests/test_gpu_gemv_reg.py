@@ -1,6 +1,7 @@
 """GPU parity of the register-operand GEMV (csrc/gemv_reg.cuh: gs = 2, up to 64 rows) at the sizes where it can go wrong:
 one and a few K blocks (four to a ring stage, two teams), ragged tiles of 256 columns, the edges of the eight-row
-n-tiles, matrices that one thread block covers and matrices that many share -- against the float64 oracle."""
+n-tiles, matrices that one thread block covers and matrices that many share -- against the float64 oracle.  Up to 16 rows
+matrices of one wave are the direct kernels': cabi.pipelined() keeps them here."""
 
 import numpy as np
 import pytest
@@ -22,11 +23,14 @@ def _case(rng, OUT, K, u, M):
 @pytest.mark.parametrize("u", (2, 3, 4))
 @pytest.mark.parametrize("M,OUT,K", [(1, 16, 32), (8, 240, 96), (9, 256, 160), (16, 272, 4096), (17, 528, 288), (31, 16, 8224),
                                      (32, 1040, 1312), (33, 256, 128),
-                                     (33, 144, 96), (61, 400, 8224), (64, 1040, 544), (65, 128, 64)])
+                                     (33, 144, 96), (61, 400, 8224), (64, 1040, 544), (65, 128, 64),
+                                     (5, 272, 4096), (8, 528, 288), (7, 1040, 1312), (5, 9616, 32), (8, 9616, 544), (9, 9616, 96),
+                                     (16, 9616, 1312)])
 def test_edges(rng, u, M, OUT, K):
     import cabi
     X, p = _case(rng, OUT, K, u, M)
-    got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
+    with cabi.pipelined():
+        got, gotf = cabi.gemv("batched", cabi.bf16_dev(X), cabi.planes_to_dev(p), M=M)
     cabi.check_output(got, gotf, orc.wonly_matmul(p, X), MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
 
 
@@ -52,9 +56,10 @@ def test_misaligned_activations_and_smallest_workspace(rng, u, M):
     ws = torch.empty(full, dtype=torch.uint8, device="cuda")
     served = []
     for size in range(full, 0, -max(256, full // 64)):
-        rc = L.msaq_wonly_gemv_batched(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
-                                       pd["shared_cm"].data_ptr(), y.data_ptr(), None, M, OUT, K // 32, u, 2, ws.data_ptr(),
-                                       size, torch.cuda.current_stream().cuda_stream)
+        with cabi.pipelined():
+            rc = L.msaq_wonly_gemv_batched(x.data_ptr(), pd["scale_exp"].data_ptr(), pd["upper_cm"].data_ptr(),
+                                           pd["shared_cm"].data_ptr(), y.data_ptr(), None, M, OUT, K // 32, u, 2, ws.data_ptr(),
+                                           size, torch.cuda.current_stream().cuda_stream)
         if rc:
             assert rc == -3
             break
@@ -63,15 +68,16 @@ def test_misaligned_activations_and_smallest_workspace(rng, u, M):
         assert orc.rel_fro(s, got) < 1e-3           # a few roundings to bf16 at most
 
 
-def test_bits_do_not_depend_on_the_workspace_contents(rng):
+@pytest.mark.parametrize("u,M,OUT,K", [(3, 5, 1024, 2048), (4, 8, 10256, 1056), (2, 12, 7120, 1056), (4, 40, 1040, 2048)])
+def test_bits_do_not_depend_on_the_workspace_contents(rng, u, M, OUT, K):
     import cabi
-    X, p = _case(rng, 1024, 2048, 3, 5)
+    X, p = _case(rng, OUT, K, u, M)
     pd = cabi.planes_to_dev(p)
     x = cabi.bf16_dev(X)
-    first = cabi.gemv("batched", x, pd, M=5)[1]
-    junk = torch.randint(0, 255, (64 << 20,), dtype=torch.uint8, device="cuda")
-    del junk                                        # the next workspace comes out of these bytes
-    assert np.array_equal(cabi.gemv("batched", x, pd, M=5)[1], first)
+    with cabi.pipelined():
+        first = cabi.gemv("batched", x, pd, M=M, fill=0)[1]
+        for fill in (0xFF, 0x5A, 0x7F):
+            assert np.array_equal(cabi.gemv("batched", x, pd, M=M, fill=fill)[1], first)
 
 
 @pytest.mark.parametrize("u,M", [(3, 2), (4, 12), (4, 50)])
@@ -87,7 +93,8 @@ def test_wait_gives_up_and_next_call_is_correct(rng, u, M):
         _, gotf = cabi.gemv("batched", x, pd, M=M)
     assert _status() & 1
     assert np.isnan(gotf).any()
-    got2, gotf2 = cabi.gemv("batched", x, pd, M=M)
+    with cabi.pipelined():
+        got2, gotf2 = cabi.gemv("batched", x, pd, M=M)
     cabi.check_output(got2, gotf2, ref, MAX_ABS_REL_TOL, REL_FRO_TOL, F32_REL_FRO_TOL)
     assert _status() == 0
 
