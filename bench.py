@@ -51,7 +51,7 @@ def parse():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--batch", type=int, default=1)
     ap.add_argument("--no-detail", action="store_true")
-    ap.add_argument("--case", default=None, choices=["gemv", "gemv16", "kv", "layer"],
+    ap.add_argument("--case", default=None, choices=["gemv", "gemv16", "gemv128", "small", "pack", "kv", "layer"],
                     help="run a few launches of one op only (small driver for ncu captures)")
     a = ap.parse_args()
     if a.steps is None:
@@ -494,7 +494,7 @@ def run_ours(args):
         "n_gpus": world, "steps": args.steps, "warmup": max(3, args.warmup),
         "ms_per_step": round(ms_per_step, 5), "us_per_step": round(ms_per_step * 1e3, 2),
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "u4 codes -> int8 MMA (M<=8) / bf16 tcgen05 (M>=9), fp32 accumulate, bf16 in/out", "data": "synthetic",
+        "dtype": "u4 codes -> int8 MMA (M<=4, large M<=8) / exact bf16 MMA (above, tcgen05 for the largest batches), fp32 accumulate, bf16 in/out", "data": "synthetic",
         "config": {
             "workload": "llama-3.1-70b-shaped decoder layer, one decode step (RoPE on q and k included), u4/gs2 packed "
                         "weights and KV cache, hidden 8192, Hq 64, Hkv 8, D 128, FFN 28672, Lk %d, B %d" % (LK, B),
@@ -815,8 +815,9 @@ def run_reference(args):
 
 
 def run_case(args):
-    """A handful of launches of one op on cuda:0: the 28672x4096 u4/gs2 GEMV with one row or sixteen (92 MB per
-    launch) or the GQA 32/8 flash-decode at Lk=16384, B=8 (157 MB per launch).  Meant to be run under ncu."""
+    """A handful of launches of one op on cuda:0: the 28672x4096 u4/gs2 GEMV with one, 16 or 128 rows (92 MB per launch), the
+    GEMVs of one wave (4096x14336 with one row and with eight, 46 MB), loading (packing 14336x4096, a prompt of 8 x 8191 keys, widening
+    4096x14336 to bf16), the GQA 32/8 flash-decode at Lk=16384, B=8 (157 MB) or the layer step.  Meant to be run under ncu."""
     import torch
     from ms_kernel_b200 import ops
     dev = torch.device("cuda", 0)
@@ -831,9 +832,24 @@ def run_case(args):
         torch.cuda.synchronize()
         for i in range(3):
             y = sets[i % 2].eager()
-    elif args.case in ("gemv", "gemv16"):
+    elif args.case == "small":
+        lins = [make_linear(4096, 14336, U, GS, 3 + i, dev) for i in range(4)]
+        x = torch.randn((8, 14336), generator=g, device=dev).to(torch.bfloat16)
+        for i in range(12):                                 # integer and bf16 direct kernels in turn
+            y = lins[i % 4].fwd(x[0] if i & 1 else x)
+    elif args.case == "pack":
+        from ms_kernel_b200 import pack
+        W = (torch.randn((14336, 4096), generator=g, device=dev) * 0.02).to(torch.bfloat16)
+        K, V = (torch.randn((1, 8, 8191, 128), generator=g, device=dev).to(torch.bfloat16) for _ in range(2))
+        cache = ops.KVCache(1, 8, 128, 8192, U, GS, dev, rotate=True)
+        lins = [make_linear(4096, 14336, U, GS, 3 + i, dev) for i in range(3)]
+        for lin in lins:
+            p = pack.pack_weight(W, U, GS, device=dev)
+            cache.fill(K, V)
+            y = torch.ops.msaq.ms_dequant_bf16(lin.scale_exp, lin.upper_cm, lin.shared_cm, lin.OUT, lin.K, lin.nb, lin.u, lin.gs)
+    elif args.case in ("gemv", "gemv16", "gemv128"):
         lins = [make_linear(28672, 4096, U, GS, 3 + i, dev) for i in range(4)]
-        M = 1 if args.case == "gemv" else 16               # 16 rows: the tcgen05 / tensor-memory kernel
+        M = {"gemv": 1, "gemv16": 16, "gemv128": 128}[args.case]      # integer MMA, register operands, tcgen05 / tensor memory
         x = torch.randn((M, 4096) if M > 1 else (4096,), generator=g, device=dev).to(torch.bfloat16)
         for i in range(6):
             y = lins[i % 4].fwd(x)

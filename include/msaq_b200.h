@@ -53,11 +53,12 @@ unsigned long long msaq_launch_count(void);
  *   launched with programmatic stream serialisation, so the launch and prologue of one kernel overlap the
  *   tail of the kernel before it.  Results do not change: every kernel waits for its predecessor before it
  *   reads or writes anything another kernel produces or consumes.
- * MSAQ_OPT_TENSOR_MEMORY (default 1): batched GEMVs (u=4, gs=2, 9 rows and more) run on exact bf16 operands -- up to
- *   64 rows with warp-level MMAs on register operands, above (and for large matrices from 33) on the tcgen05 tensor cores
- *   with accumulators in tensor memory; 0 keeps them on the warp-level integer MMA path (the paths agree to the output tolerance, not bit for bit).
- * MSAQ_OPT_INKERNEL_STAGING (default 1): small integer-MMA GEMVs (up to four rows, no fused prologue, at most
- *   eighteen K blocks per thread block) convert their activations inside the main kernel, one launch per GEMV; 0
+ * MSAQ_OPT_TENSOR_MEMORY (default 1): GEMVs at gs=2 with u=2 and 3, and with u=4 from nine rows on (without a prologue from five, but
+ *   for the largest matrices) run on exact bf16 operands -- up to 64 rows with warp-level MMAs on register operands, above (and for
+ *   large matrices from 33) on the tcgen05 tensor cores with accumulators in tensor memory; 0 keeps u=4 on the warp-level integer
+ *   MMA path and the others on the generic kernel (the paths agree to the output tolerance, not bit for bit).
+ * MSAQ_OPT_INKERNEL_STAGING (default 1): small pipelined integer-MMA GEMVs (up to four rows, no fused prologue, at most
+ *   eighteen K blocks per thread block, columns beyond one wave of the direct kernels) convert their activations inside the main kernel, one launch per GEMV; 0
  *   runs the separate staging kernel in front, as all other launches do.  Same staged values either way.
  * MSAQ_OPT_WAIT_POLLS (default 2^20): poll limit of every wait on a shared-memory barrier inside the pipelined
  *   kernels.  A wait that reaches it gives up: the kernel finishes by itself, the outputs the wait fed become
@@ -175,8 +176,8 @@ int msaq_wonly_gemv_fused(const void* x, int prologue, const void* addend, int a
  *   - All calls on one device share the array and it keeps the previous call's contents: the
  *     kernels reset the words that must start at zero, but two calls that overlap on the GPU
  *     (different streams, or graphs replayed concurrently) race on it.  Serialise them.
- *   - A problem whose scratch need (msaq_wonly_gemv_workspace(1, OUT, NB, u, gs)) exceeds the
- *     array is refused with MSAQ_ERR_WORKSPACE; nothing is launched.
+ *   - A problem whose scratch need (msaq_wonly_gemv_workspace(1, OUT, NB, u, gs), less what only makes some sizes faster)
+ *     exceeds the array is refused with MSAQ_ERR_WORKSPACE; nothing is launched.
  * This entry point has no counterpart in the reference.
  */
 #define MSAQ_STATIC_SCRATCH_BYTES (8u << 20)
@@ -387,9 +388,10 @@ int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps, const int8
  * every rank's exchange buffer (its own included) instead of into local memory, so the partial sums cross NVLink
  * tile by tile while the GEMV still runs; msaq_peer_exchange(partial = NULL, ...) with the same parity and
  * n = M * OUT then completes the sum.  Same arguments as msaq_wonly_gemv_fused without y / y_f32, same peer buffers
- * and parity rule as msaq_peer_exchange.  Built into the integer-MMA kernel only (u = 4, gs = 2, M <= 8, aligned
+ * and parity rule as msaq_peer_exchange.  Built into the direct and the integer-MMA kernels only (u = 4, gs = 2, M <= 8, aligned
  * column-major planes, M * OUT a multiple of 4): MSAQ_ERR_UNSUPPORTED otherwise, and the caller runs the two calls
- * separately.
+ * separately.  (At five to eight rows the GEMV without the push may run on the register-operand kernel, whose sums agree with
+ * these to the output tolerance.)
  */
 int msaq_wonly_gemv_fused_push(const void* x, int prologue, const void* addend, int addend_is_f32, float eps,
                                void* h_out, const int8_t* scale_exp, const uint8_t* upper_cm,

@@ -335,7 +335,7 @@ int launch_xprep(const XprepArgs& xa, int mode, unsigned grid, cudaStream_t st) 
 // whole of K.  So the model's cycles are held against what the pipelined kernel's time grows with: the bytes, and K where the
 // staging kernel adds and takes a norm.  Matrices so narrow that that kernel's tiles are at their narrowest never cross below the
 // limits.  us, pipelined -> direct:
-//   plain     3 rows   4096x14336 22.0 -> 19.3   5120x14336 24.4 -> 32.0
+//   plain     3 rows   4096x14336 21.8 -> 19.3   5120x14336 24.4 -> 32.0
 //   silu      1 row    4096x14336 20.7 -> 15.3   5120x14336 23.2 -> 24.1
 //             3 rows   4096x4096 13.6 -> 10.9    8192x4096 18.4 -> 16.6   4096x14336 22.5 -> 28.3   5120x14336 24.0 -> 49.6
 //   add+norm  2 rows   4096x14336 27.8 -> 23.0   5120x11008 23.8 -> 29.8
@@ -373,7 +373,8 @@ int run_direct(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, co
 int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh,
             void* Y, float* Yf, int64_t M, int64_t OUT, int64_t NB, void* ws, cudaStream_t st, int fmt = GF_MSAQ_U4,
             const PeerPush* push = nullptr, const void* res = nullptr) {
-    // (five rows and more without a prologue: as gemv_dispatch chooses, so that a residual add or a push changes no bit)
+    // (five rows and more without a prologue: the direct kernel where gemv_dispatch takes it; the sizes that it gives to the
+    // register kernel come here only with a push, which that kernel does not have)
     int cg = 1, cs = 1;
     if (fmt == GF_MSAQ_U4 && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4, &cg, &cs))
         return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, cg, cs, push, res, st);

@@ -13,8 +13,8 @@
 //   * the code q * 2^e is exact in bf16 (see gr_decode_row), so products are exact in fp32 and one accumulator runs over
 //     the thread block's whole K range: no work per 32-block behind the MMA;
 //   * one thread block per SM, on the schedule and the per-warp tile hand-off of gemv_mma.cuh.
-// Measured (28672 x 4096, u = 4, 16 rows: 52.2 -> 38.5 us, of which copies and fixed costs alone take 22 us): ALU 38, FMA 34
-// and 96 instructions in all per 16 x 32 weights.  Copies of a stage are issued by lanes in one instruction, four K blocks
+// Measured (28672 x 4096, u = 4, 16 rows: 52.2 -> 37.4 us, of which copies and fixed costs alone take 22 us): 88 instructions in
+// all per 16 x 32 weights, ALU pipe 44 % and FMA pipe 37 % busy.  Copies of a stage are issued by lanes in one instruction, four K blocks
 // to a stage: a copy-issuing warp spends about 0.4 us on a stage whatever its size (two K blocks: 41.6 us), which is also
 // why each team has its own (one for both: 42.4 us).
 //
@@ -26,7 +26,8 @@
 namespace msaq {
 
 constexpr int GR_MAX_M = 64;                       // activation rows per launch
-// 128-column groups per tile, by n-tiles of eight activation rows: as many as the accumulators leave registers for
+// 128-column groups per tile, by n-tiles of eight activation rows.  Eighteen warps leave a thread 96 registers: one and two n-tiles fit
+// with two groups, four n-tiles (17 to 32 rows) spill 240 to 300 bytes of it, eight, with one group, 20 to 60.
 __host__ __device__ constexpr int gr_groups_of(int mt) { return mt <= 4 ? 2 : 1; }
 __host__ __device__ constexpr int gr_tc(int mt) { return gr_groups_of(mt) * GM_GROUP; }
 constexpr int GR_KB = 4;                           // K blocks per ring stage

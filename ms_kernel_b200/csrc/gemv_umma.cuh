@@ -1,6 +1,7 @@
 // Weight-only GEMV on the fifth-generation tensor cores, Y[M][OUT] = X[M][K] * dequant(W)^T, in
 // tiles of up to 128 activation rows: u = 4, gs = 2 from nine rows up, and the 5+3 and 6+2 bit
-// formats (u = 3, u = 2 at gs = 2) at every batch size.
+// formats (u = 3, u = 2 at gs = 2) at every batch size.  (Batches up to 64 rows come here where the register kernel is the slower
+// one, see reg_serves() in gemv.cu, and where X is misaligned or the workspace too small for the others.)
 //
 // At these batch sizes the work is a real contraction, so it goes to tcgen05.mma with the
 // accumulator in tensor memory.  The weights stay packed in HBM (25 to 29 bytes per 32-block)

@@ -62,9 +62,9 @@ int current_device();         // -1 if the runtime cannot say
 int sm_count();               // SM count of the current device (cached per device)
 int require_sm100();          // MSAQ_OK or MSAQ_ERR_DEVICE
 bool option_chained_launch(); // kernels are launched with programmatic stream serialisation
-bool option_tensor_memory();  // batched GEMVs of 9 rows and more run on tcgen05 with tensor-memory accumulators
+bool option_tensor_memory();  // MSAQ_OPT_TENSOR_MEMORY: GEMVs of u = 2, 3 and of five rows and more on exact bf16 operands
 bool option_early_weights();   // MSAQ_OPT_EARLY_WEIGHTS: weights are fetched before the wait on the kernel in front
-bool option_inkernel_staging(); // GEMVs of up to four rows stage their activations inside the main kernel
+bool option_inkernel_staging(); // pipelined GEMVs of up to four rows stage their activations inside the main kernel
 unsigned option_wait_polls(); // poll limit of the bounded mbarrier waits
 int option_test_skip_stage(); // test hook: pipeline stage whose copy the first CTA's producer leaves out (-1: none)
 int* sticky_status();         // device address of the per-device status word on the current device (null on failure)
