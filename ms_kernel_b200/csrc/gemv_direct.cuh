@@ -350,14 +350,14 @@ gemv_direct_bf16_kernel(const GemvDirectArgs a) {
     constexpr int HALVES = MT > 1 ? 2 : 1, WARPS = GD_WARPS / HALVES;        // 16 rows: half of the warps add theirs to the others'
     __shared__ float red[WARPS][ROWS][COLS];
     __shared__ float part[ROWS * COLS];
-    __shared__ uint32_t consts[GrConst<U>::N];
+    __shared__ __align__(16) uint32_t consts[GrConst<U>::N];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int stride = GD_WARPS * a.cs, tile = blockIdx.x / a.cs, c0 = tile * COLS;
     const int first = (a.cs > 1 ? (int)cluster_rank() : 0) * GD_WARPS + warp;
     const int ngroups = min(CG, (a.OUT - c0) >> 4);
     const GrLane ln = gr_lane<U>(t);
-    if (tid < GrConst<U>::N) consts[tid] = GrConst<U>::value(tid);
+    if (tid == 0) GrConst<U>::store(consts);
 
     const int64_t col = (int64_t)first * a.OUT + c0 + g;
     const uint8_t* pu = a.upper_cm + col * UB + ln.up_off;

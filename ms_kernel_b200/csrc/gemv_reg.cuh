@@ -91,7 +91,7 @@ struct GrConst {
     static constexpr int WB = 8 - U;
     static constexpr int N = 9;
     uint32_t um, ux, sm, sx, uoff, soff, two_u, one, neg0;
-    __device__ static __forceinline__ uint32_t value(int i) {
+    __device__ static __forceinline__ constexpr uint32_t value(int i) {
         switch (i) {
             case 0: return ((1u << WB) - 1u) * 0x00010001u;                          // an upper code in each half
             case 1: return 0x43004300u | (0x00010001u << (WB - 1));                  // bf16 128.0, and the code's sign bit
@@ -103,6 +103,11 @@ struct GrConst {
             case 7: return 0x3F803F80u;
             default: return 0x80008000u;                                             // -0: the neutral addend
         }
+    }
+    // by one thread, all of them immediates (a thread per constant looks its own up in constant memory: 0.1 us of a launch)
+    __device__ static __forceinline__ void store(uint32_t* consts) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) consts[i] = value(i);
     }
     __device__ __forceinline__ explicit GrConst(uint32_t a) {
         uint32_t* const v[N] = {&um, &ux, &sm, &sx, &uoff, &soff, &two_u, &one, &neg0};
@@ -285,7 +290,7 @@ gemv_reg_kernel(const GemvRegArgs a) {
     __shared__ __align__(8) uint64_t bar_full_all[GR_TEAMS * GM_MAX_STAGES];
     __shared__ __align__(8) uint64_t bar_empty_all[GR_TEAMS * GM_MAX_STAGES];
     __shared__ unsigned int marker_sh[GM_WARPS];
-    __shared__ uint32_t consts[GrConst<U>::N];
+    __shared__ __align__(16) uint32_t consts[GrConst<U>::N];
 
     constexpr int UB = gr_ub(U), SB = gr_sb(U), GR_GROUPS = gr_groups_of(MT), GR_TC = gr_tc(MT);
     constexpr int OFF_SH = GR_TC * UB, OFF_SC = GR_TC * (UB + SB), SUB = gr_sub_bytes(U, MT), OFF_X = GR_KB * SUB;
@@ -302,7 +307,7 @@ gemv_reg_kernel(const GemvRegArgs a) {
     uint64_t* const bar_full = bar_full_all + team * sch.stages;
     uint64_t* const bar_empty = bar_empty_all + team * sch.stages;
 
-    if (tid < GrConst<U>::N) consts[tid] = GrConst<U>::value(tid);
+    if (tid == 32) GrConst<U>::store(consts);
     if (tid == 0) {
         for (int s = 0; s < GR_TEAMS * sch.stages; ++s) {
             mbar_init(smem_u32(&bar_full_all[s]), 1 + 32);       // the bulk copies' transaction, and the lanes' own copies
