@@ -236,13 +236,13 @@ struct RegPlan {
 //     6144x4096 31.8 -> 24.8 | 34.3 -> 25.2 | 40.1 -> 25.8     5120x8192 37.6 -> 33.9 | 43.0 -> 34.4 | 47.1 -> 35.1
 //     14336x3072 33.1 -> 35.7 | 37.7 -> 36.6 | 42.4 -> 37.8    4096x14336 41.8 -> 43.9 | 44.3 -> 44.5 | 48.6 -> 44.8
 //     14336x4096 37.8 -> 43.3 | 42.4 -> 44.5 | 47.1 -> 45.7    57344x512 31.9 -> 33.3 | 36.9 -> 35.1 | 43.3 -> 37.4
-//     u3: 42272x1088 at 54 rows 46.6 -> 49.4, 14336x4096 at 64 rows 49.2 -> 50.2
+//     56 rows: 14880x3072 41.1 -> 37.6, 14336x4096 44.5 -> 45.5;  u3: 42272x1088 at 54 rows 46.6 -> 49.4, 14336x4096 at 64 rows 49.2 -> 50.2
 bool reg_serves(int64_t M, int64_t OUT, int64_t NB, int u) {
     const int64_t bytes = OUT * NB * (gr_ub(u) + gr_sb(u) + 1), weights = OUT * NB * BLOCK;
     if (M > GR_MAX_M || (M > 16 && u == 3 && bytes > (300LL << 20))) return false;
     if (M > 32) {
         const bool wide = OUT >= 14000;
-        const int64_t millions = M <= 40 ? (wide ? 30 : 52) : M <= 48 ? (wide ? 40 : 60) : !wide ? 70 : M <= 56 || u == 3 ? 45 : 60;
+        const int64_t millions = M <= 40 ? (wide ? 31 : 52) : M <= 48 ? (wide ? 40 : 60) : !wide ? 70 : u == 3 ? 45 : M <= 56 ? 52 : 60;
         if (bytes > (48LL << 20) || weights > millions * 1000000) return false;
     }
     return u != 4 || M >= GU_MIN_M || (M >= 5 && bytes <= (100LL << 20));

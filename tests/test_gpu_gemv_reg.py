@@ -127,7 +127,7 @@ def test_largest_finite_weights(rng, u, M, OUT, K):
 
 
 @pytest.mark.parametrize("u,M,OUT,K,launches", [(4, 33, 6144, 4096, 2), (4, 33, 4096, 11008, 2), (4, 33, 14336, 3072, 3), (4, 40, 4096, 14336, 3),
-                                                (4, 44, 14336, 2048, 2), (4, 48, 4096, 14336, 2), (4, 48, 14336, 3072, 3), (4, 49, 14336, 4096, 3),
+                                                (4, 44, 14336, 2048, 2), (4, 48, 4096, 14336, 2), (4, 48, 14336, 3072, 3), (4, 49, 14336, 4096, 3), (4, 56, 14880, 3072, 2),
                                                 (4, 64, 14336, 4096, 2), (4, 64, 57344, 512, 2), (3, 37, 47056, 256, 2), (3, 54, 42272, 1088, 3),
                                                 (3, 64, 12288, 4096, 2), (3, 64, 14336, 4096, 3), (2, 36, 57344, 512, 2), (2, 36, 28672, 1536, 3),
                                                 (2, 17, 57344, 512, 2)])
