@@ -129,6 +129,8 @@ int msaq_wonly_gemv_wide(const void* x, const int8_t* scale_exp, const uint8_t* 
  * (The tensor-memory kernel widens q * 2^e through an fp32 constant of about 2^23 * 2^e: block exponents above 104 overflow
  * there.  bf16 weights of magnitude below 2^110 never produce them.  It serves gs = 2 from 33 rows on, and fewer rows -- u = 4
  * from nine, u = 2 and 3 from one -- where X is not 16-byte aligned or the workspace is smaller than the query says.)
+ * Y may be X's own memory (OUT == K), here and with the prologues below: such a call runs on kernels that have staged the
+ * activations before they store a result.
  * Replaces op `msaq::wonly_gemv_batched` (csrc/pybind.cpp:205-206, host
  * csrc/w_gemv.cu:1514-1570).
  */

@@ -18,6 +18,16 @@ int gemv_run_generic(const __nv_bfloat16* X, const int8_t* se, const uint8_t* up
                      cudaStream_t st);
 namespace {
 
+// Whether a call writes its outputs over its inputs.  The staging kernels have read all of the activations when the main kernel
+// starts, so those paths may; the kernels that read activations while others of their thread blocks store results may not.
+bool overlap(const void* a, int64_t na, const void* b, int64_t nb) {
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);
+    return a && b && a0 < b0 + (uintptr_t)nb && b0 < a0 + (uintptr_t)na;
+}
+bool in_place(const void* in, int64_t in_bytes, const void* Y, const float* Yf, int64_t outputs) {
+    return overlap(in, in_bytes, Y, outputs * 2) || overlap(in, in_bytes, Yf, outputs * 4);
+}
+
 // ---- tuned path (u4/gs2, column-major planes, OUT % 16 == 0) --------------------
 struct MmaPlan {
     GemvSchedule sch;        // sch.nb counts units of `kb` K blocks
@@ -372,11 +382,11 @@ int run_direct(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, co
 
 int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const uint8_t* up, const uint8_t* sh,
             void* Y, float* Yf, int64_t M, int64_t OUT, int64_t NB, void* ws, cudaStream_t st, int fmt = GF_MSAQ_U4,
-            const PeerPush* push = nullptr, const void* res = nullptr) {
+            const PeerPush* push = nullptr, const void* res = nullptr, bool over_inputs = false) {
     // (five rows and more without a prologue: the direct kernel where gemv_dispatch takes it; the sizes that it gives to the
     // register kernel come here only with a push, which that kernel does not have)
     int cg = 1, cs = 1;
-    if (fmt == GF_MSAQ_U4 && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4, &cg, &cs))
+    if (fmt == GF_MSAQ_U4 && !over_inputs && (M <= 4 || (pro.mode == XP_PLAIN && option_tensor_memory())) && direct_usable(X, pro.mode, M, OUT, NB, 4, &cg, &cs))
         return run_direct(X, pro, se, up, sh, Y, Yf, M, OUT, NB, 4, cg, cs, push, res, st);
     const MmaPlan p = plan_mma(M, OUT, NB, fmt);
     uint8_t* base = static_cast<uint8_t*>(ws);
@@ -411,7 +421,7 @@ int run_mma(const __nv_bfloat16* X, const Prologue& pro, const int8_t* se, const
         const long long max_iter = (sch.units() + sch.grid - 1) / sch.grid;
         const long long table = max_iter * p.kb * GM_XREC;
         const bool in_kernel = fmt == GF_MSAQ_U4 && passes == 1 && pro.mode == XP_PLAIN && option_inkernel_staging() &&
-                               table <= GM_MAX_TABLE;
+                               !over_inputs && table <= GM_MAX_TABLE;
         if (in_kernel) {
             const int per_sm = (sch.grid + sm_count() - 1) / sm_count();
             int stages = (200 * 1024 / per_sm - (int)table) / (p.kb * gm_stage_bytes(sch.tc, passes, fmt));
@@ -475,18 +485,20 @@ int gemv_dispatch(const void* X, const int8_t* se, const uint8_t* up, const uint
     // the tensor-memory epilogue stores 16 outputs at a time: Y (and Y_f32) must be 16-byte aligned for it
     const bool tm_ok = aligned && umma_eligible(OUT, u, gs, cm) && option_tensor_memory() &&
                        !((reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(Yf)) & 15);
+    const bool over_inputs = in_place(X, M * NB * BLOCK * 2, Y, Yf, M * OUT);
     int cg = 1, cs = 1;
-    if (tm_ok && direct_usable(X, XP_PLAIN, M, OUT, NB, u, &cg, &cs))
+    if (tm_ok && !over_inputs && direct_usable(X, XP_PLAIN, M, OUT, NB, u, &cg, &cs))
         return run_direct(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, u, cg, cs, nullptr, nullptr, st);
     RegPlan reg;
-    if (reg_usable(X, se, up, sh, Y, Yf, M, OUT, NB, u, gs, cm, ws, ws_bytes, &reg))
+    if (!over_inputs && reg_usable(X, se, up, sh, Y, Yf, M, OUT, NB, u, gs, cm, ws, ws_bytes, &reg))
         return run_reg(x, se, up, sh, Y, Yf, M, OUT, NB, u, reg, ws, st);
     // u = 4 keeps up to eight rows on the integer-MMA kernel
     if (tm_ok && (u != 4 || M >= GU_MIN_M)) return run_umma(x, se, up, sh, Y, Yf, M, OUT, NB, u, ws, st);
     // the integer-MMA kernel's finishing warps store four outputs at a time: 8-byte aligned bf16, 16-byte aligned fp32
     const bool out_ok = !((reinterpret_cast<uintptr_t>(Y) & 7) | (reinterpret_cast<uintptr_t>(Yf) & 15));
     if (mma_usable(se, up, sh, ws, OUT, u, gs, cm) && out_ok)
-        return run_mma(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, ws, st);
+        return run_mma(x, Prologue{XP_PLAIN, nullptr, 0, nullptr, 0.0f}, se, up, sh, Y, Yf, M, OUT, NB, ws, st, GF_MSAQ_U4, nullptr,
+                       nullptr, over_inputs);
 
     return gemv_run_generic(x, se, up, sh, Y, Yf, M, OUT, NB, f, cm, static_cast<uint8_t*>(ws) + WS_CTL_BYTES, st);
 }
@@ -602,8 +614,10 @@ extern "C" int msaq_wonly_gemv_fused(const void* x, int prologue, const void* ad
     const bool small = M < GU_MIN_M || !option_tensor_memory();
     if (mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true) && vec_ok && small) {
         const Prologue pro{prologue, addend, addend_is_f32, h_out, eps};
+        const bool over_inputs = in_place(x, M * K * (prologue == MSAQ_PRO_SILU_MUL ? 4 : 2), y, y_f32, M * OUT) ||
+                                 in_place(addend, M * K * (addend_is_f32 ? 4 : 2), y, y_f32, M * OUT);
         return run_mma(static_cast<const __nv_bfloat16*>(x), pro, scale_exp, upper_cm, shared_cm, y, y_f32, M, OUT, NB,
-                       workspace, st);
+                       workspace, st, GF_MSAQ_U4, nullptr, nullptr, over_inputs);
     }
     // Other formats: the glue runs as kernels of its own into the tail of the workspace.
     void* tmp = static_cast<uint8_t*>(workspace) + g;
@@ -640,19 +654,20 @@ extern "C" int msaq_wonly_gemv_fused_add(const void* x, int prologue, float eps,
                     mma_usable(scale_exp, upper_cm, shared_cm, workspace, OUT, u, gs, true);
     if (ok) {
         // without a prologue the sum is the plain GEMV's, whichever kernel that is
+        const bool over_inputs = in_place(x, M * NB * BLOCK * (prologue == MSAQ_PRO_SILU_MUL ? 4 : 2), y, nullptr, M * OUT);
         int cg, cs;
         RegPlan reg;
-        if (prologue == MSAQ_PRO_NONE && M > 4 && !direct_usable(x, XP_PLAIN, M, OUT, NB, u, &cg, &cs) &&
+        if (prologue == MSAQ_PRO_NONE && M > 4 && !over_inputs && !direct_usable(x, XP_PLAIN, M, OUT, NB, u, &cg, &cs) &&
             reg_usable(x, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, u, gs, true, workspace, workspace_bytes, &reg))
             return run_reg(xb, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, u, reg, workspace, st, residual);
         const Prologue pro{prologue, nullptr, 0, nullptr, eps};
-        return run_mma(xb, pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, workspace, st, GF_MSAQ_U4, nullptr, residual);
+        return run_mma(xb, pro, scale_exp, upper_cm, shared_cm, y, nullptr, M, OUT, NB, workspace, st, GF_MSAQ_U4, nullptr, residual,
+                       over_inputs);
     }
     // Every other format and size: the same two steps as separate kernels (identical roundings).  With the residual in y's own
     // memory the product goes to the end of the workspace first.
-    const uintptr_t y0 = reinterpret_cast<uintptr_t>(y), r0 = reinterpret_cast<uintptr_t>(residual), n = (uintptr_t)M * OUT * 2;
     void* product = y;
-    if (y0 < r0 + n && r0 < y0 + n) {
+    if (overlap(y, M * OUT * 2, residual, M * OUT * 2)) {
         front = gemv_workspace_front(M, OUT, NB, u, gs, tail + product_tail(M, OUT), workspace_bytes);
         if (workspace_bytes < front + tail + product_tail(M, OUT))
             return fail(MSAQ_ERR_WORKSPACE, "workspace of %zu bytes needed for a residual add in place, %zu given",

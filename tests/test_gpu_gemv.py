@@ -300,3 +300,48 @@ def test_residual_add_in_the_residuals_own_memory(u, gs, M, OUT, K, prologue):
     assert rc == 0 and torch.equal(got, want)
     rc, got = in_place(1024)                       # too little: refused, nothing touched
     assert rc == -3 and torch.equal(got, res)
+
+
+@pytest.mark.parametrize("u,gs,M,N,prologue,launches", [(4, 2, 1, 1024, 0, 2), (4, 2, 4, 512, 0, 2), (4, 2, 1, 10240, 0, 2), (4, 2, 8, 1024, 0, 2),
+                                                        (4, 2, 6, 10240, 0, 2), (4, 2, 12, 1024, 0, 3), (4, 2, 70, 512, 0, 3), (3, 2, 3, 512, 0, 3),
+                                                        (4, 4, 2, 96, 0, 2), (4, 2, 2, 1024, 1, 2), (4, 2, 4, 1024, 3, 2), (4, 2, 8, 1024, 1, 2)])
+def test_result_over_the_activations(rng, u, gs, M, N, prologue, launches):
+    """y in x's (or the addend's) own memory: a kernel that has staged the activations first runs, and the result is that of
+    separate buffers to the rounding of the sums."""
+    from ms_kernel_b200 import _lib, ops, pack
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(N + M + u)
+    lin = ops.PackedLinear(pack.pack_weight((torch.randn((N, N), generator=g, device="cuda") * 0.02).to(torch.bfloat16), u, gs), "cuda")
+    x = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16)
+    d = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16) if prologue == 3 else None
+    want = lin.fwd(x) if prologue == 0 else lin.fwd_fused(x, prologue, d)
+    want = want[0] if prologue == 3 else want
+    buf = (d if prologue == 3 else x).clone()
+    h = torch.empty_like(x)
+    wsb = L.msaq_wonly_gemv_fused_workspace(M, N, N // 32, u, gs)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    n0 = L.msaq_launch_count()
+    _lib.check(L.msaq_wonly_gemv_fused((x if prologue == 3 else buf).data_ptr(), prologue, buf.data_ptr() if prologue == 3 else None, 0, 1e-5,
+                                       h.data_ptr(), lin.scale_exp.data_ptr(), lin.upper_cm.data_ptr(), lin.shared_cm.data_ptr(), buf.data_ptr(),
+                                       None, M, N, N // 32, u, gs, ws.data_ptr(), wsb, torch.cuda.current_stream().cuda_stream))
+    assert L.msaq_launch_count() - n0 == launches
+    torch.cuda.synchronize()
+    assert orc.rel_fro(buf.float().cpu().numpy(), want.float().cpu().numpy()) < REL_FRO_TOL
+
+
+@pytest.mark.parametrize("M,N,prologue", [(1, 1024, 1), (4, 512, 0), (6, 10240, 0), (8, 1024, 0), (12, 512, 1)])
+def test_residual_stream_updated_in_place(rng, M, N, prologue):
+    """x, the residual and y all one buffer: h <- h + W pro(h)."""
+    from ms_kernel_b200 import _lib, ops, pack
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    lin = ops.PackedLinear(pack.pack_weight((torch.randn((N, N), generator=g, device="cuda") * 0.02).to(torch.bfloat16), 4, 2), "cuda")
+    h = torch.randn((M, N), generator=g, device="cuda").to(torch.bfloat16)
+    want = lin.fwd_fused_add(h, prologue, h)
+    wsb = L.msaq_wonly_gemv_fused_workspace(M, N, N // 32, 4, 2)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    _lib.check(L.msaq_wonly_gemv_fused_add(h.data_ptr(), prologue, 1e-5, lin.scale_exp.data_ptr(), lin.upper_cm.data_ptr(), lin.shared_cm.data_ptr(),
+                                           h.data_ptr(), h.data_ptr(), M, N, N // 32, 4, 2, ws.data_ptr(), wsb,
+                                           torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert orc.rel_fro(h.float().cpu().numpy(), want.float().cpu().numpy()) < REL_FRO_TOL
